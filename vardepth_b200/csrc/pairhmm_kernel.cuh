@@ -644,9 +644,18 @@ struct HapMeta {
 };
 constexpr int kMetaRing = 64;
 
+// Inlined into its kernel, with the kernel's parameters in the constant bank
+// (__grid_constant__): x and k2 are then constant operands of the packed FMAs.
+// What bounds the row loop is the register file's read ports: an FFMA2 of
+// three register pairs issues every 4.2 cycles, one that shares a constant
+// operand every 2.1-2.3 (measured, 16 warps per SM; the FMA pipe needs 2).  As
+// a called function it held x, k2 and the two views in registers and spilled
+// at 8 rows (204 bytes loaded): 20,000 reads of 150 / 224 / 250 bases against
+// one haplotype ran 3,807 / 4,077 / 3,818 GCUPS, inlined 4,357 / 4,874 / 4,502
+// (no spills).
 template <int R>
-__device__ __noinline__ void process_pair(const BatchView bv, const QueueView qv, const ItemRef it,
-                                          const Tables<float>* __restrict__ tb, const Scalars<float> sc,
+__device__ __forceinline__ void process_pair(const BatchView& bv, const QueueView& qv, const ItemRef& it,
+                                          const Tables<float>* __restrict__ tb, const Scalars<float>& sc,
                                           const int lane, float4* __restrict__ sv, HapMeta* __restrict__ ring) {
   constexpr unsigned FULL = 0xffffffffu;
   constexpr double kLn2 = 0.6931471805599453094;
@@ -1007,8 +1016,8 @@ pairhmm_kernel(const BatchView bv, const QueueView qv, const Tables<T>* __restri
 // registers either.)
 template <int kLoR, int kHiR, int kBlocks, int kWarps = kWarpsPerBlock>
 __global__ void __launch_bounds__(kWarps * kWarp, kBlocks)
-pairhmm_pair_kernel(const BatchView bv, const QueueView qv, const Tables<float>* __restrict__ gtab,
-                    const Scalars<float> sc) {
+pairhmm_pair_kernel(const __grid_constant__ BatchView bv, const __grid_constant__ QueueView qv,
+                    const Tables<float>* __restrict__ gtab, const __grid_constant__ Scalars<float> sc) {
   __shared__ Tables<float> tab;
   // per warp: the lane states laid down at a shared haplotype prefix
   __shared__ float4 saves[kWarps][(kHiR + 2) * kWarp];
