@@ -115,8 +115,10 @@ __host__ __device__ inline long long grad_slot_elems(int R, int m, bool store_al
 template <typename T> struct GradConsts { static constexpr int kTarget = 100, kMax = 120; };
 template <> struct GradConsts<double> { static constexpr int kTarget = 600, kMax = 900; };
 
+// Inlined so that x, k2 and the views are constant operands (40 regions: 18.4 ->
+// 17.6 ms a call).
 template <typename T, int R, bool GEN, bool ANCH>
-__device__ __noinline__ void grad_pair(const BatchView& bv, const GradView& gv, const RescueEntry item,
+__device__ __forceinline__ void grad_pair(const BatchView& bv, const GradView& gv, const RescueEntry item,
                                        const Tables<T>* __restrict__ tb, const Scalars<T>& sc,
                                        const GradTables* __restrict__ gt, const GradScalars& gs, const int lane,
                                        T* __restrict__ slot, T* __restrict__ sbuf) {
@@ -446,8 +448,9 @@ template <> struct GradMinBlocks<double> { static constexpr int value = 1; };
 
 template <typename T, bool ANCH>
 __global__ void __launch_bounds__(kWarpsPerBlock * kWarp, GradMinBlocks<T>::value)
-pairhmm_grad_kernel(const BatchView bv, const GradView gv, const Tables<T>* __restrict__ gtab,
-                    const Scalars<T> sc, const GradTables* __restrict__ gtt, const GradScalars gs) {
+pairhmm_grad_kernel(const __grid_constant__ BatchView bv, const __grid_constant__ GradView gv,
+                    const Tables<T>* __restrict__ gtab, const __grid_constant__ Scalars<T> sc,
+                    const GradTables* __restrict__ gtt, const __grid_constant__ GradScalars gs) {
   __shared__ Tables<T> tab;
   __shared__ GradTables gt;
   {

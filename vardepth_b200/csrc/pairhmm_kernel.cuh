@@ -119,9 +119,13 @@ constexpr int kDriftTries = 6;
 //    row-0 deletions D[0][j] = g x^(j-1) (anchored.cpp:9).
 constexpr uint32_t kNeverBase = 0x10000u;  // compares unequal to every base byte
 
+// Inlined, with the kernel's parameters in the constant bank (see process_pair
+// for why): 20,000 single reads of 96 / 150 bases 3,285 / 3,166 -> 3,611 /
+// 3,582 GCUPS, in FP64 of 250 bases 1,814 -> 1,936 (a lone warp 140 -> 94 ns a
+// step; the called function spilled).
 template <typename T, int R, bool GEN, bool ANCH, bool DRIFT = false>
-__device__ __noinline__ void process_item(const BatchView bv, const QueueView qv, const ItemRef it,
-                                          const Tables<T>* __restrict__ tb, const Scalars<T> sc,
+__device__ __forceinline__ void process_item(const BatchView& bv, const QueueView& qv, const ItemRef& it,
+                                          const Tables<T>* __restrict__ tb, const Scalars<T>& sc,
                                           const int lane, typename Vec2<T>::type* __restrict__ scratch) {
   using T2 = typename Vec2<T>::type;
   constexpr unsigned FULL = 0xffffffffu;
@@ -947,8 +951,8 @@ template <> struct MinBlocks<double> { static constexpr int value = 3; };
 
 template <typename T, bool ANCH>
 __global__ void __launch_bounds__(kWarpsPerBlock * kWarp, MinBlocks<T>::value)
-pairhmm_kernel(const BatchView bv, const QueueView qv, const Tables<T>* __restrict__ gtab,
-               const Scalars<T> sc, const int tier) {
+pairhmm_kernel(const __grid_constant__ BatchView bv, const __grid_constant__ QueueView qv,
+               const Tables<T>* __restrict__ gtab, const __grid_constant__ Scalars<T> sc, const int tier) {
   __shared__ Tables<T> tab;
   {
     const int words = (int)(sizeof(Tables<T>) / sizeof(int));
@@ -1059,8 +1063,8 @@ pairhmm_pair_kernel(const __grid_constant__ BatchView bv, const __grid_constant_
 // per lane have no strip-mined variant go on to FP64 unchanged.
 template <int kBlocks>
 __global__ void __launch_bounds__(kWarpsPerBlock * kWarp, kBlocks)
-pairhmm_drift_kernel(const BatchView bv, const QueueView qv, const Tables<float>* __restrict__ gtab,
-                     const Scalars<float> sc) {
+pairhmm_drift_kernel(const __grid_constant__ BatchView bv, const __grid_constant__ QueueView qv,
+                     const Tables<float>* __restrict__ gtab, const __grid_constant__ Scalars<float> sc) {
   __shared__ Tables<float> tab;
   {
     const int words = (int)(sizeof(Tables<float>) / sizeof(int));

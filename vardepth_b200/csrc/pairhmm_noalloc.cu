@@ -146,7 +146,8 @@ __global__ void na_prep_reads(const unsigned char* __restrict__ read_quals, cons
 // haplotypes, derived here instead of read from a host-built list.
 template <typename T, bool ANCH>
 __global__ void __launch_bounds__(kWarpsPerBlock * kWarp, MinBlocks<T>::value)
-na_primary(const BatchView bv, const QueueView qv, const Scalars<T> sc, int n_reads, unsigned char* scratch) {
+na_primary(const __grid_constant__ BatchView bv, const __grid_constant__ QueueView qv,
+           const __grid_constant__ Scalars<T> sc, int n_reads, unsigned char* scratch) {
   __shared__ Tables<T> tab;
   {
     const Tables<T>* g = reinterpret_cast<const Tables<T>*>(scratch + (sizeof(T) == 4 ? kOffTab32 : kOffTab64));
