@@ -143,7 +143,8 @@ typedef struct vd_tuning {
                            host work and copies of one chunk overlap the kernels of the previous
                            one; 0 = the default (300), 1e6 or more = one chunk */
   int long_mode;        /* reads longer than one strip, FP32 semiglobal: VD_LONG_WARP (default) runs a
-                           read against two haplotypes per warp with per-lane power-of-two boosts;
+                           read against two haplotypes at a time, a warp per strip, the strips of
+                           a pair side by side, lanes scaled by powers of two;
                            VD_LONG_BLOCK the same items on a block per item, whose 4 warps split
                            each strip (4x shorter latency per pair, for batches of few long
                            pairs); VD_LONG_SINGLE the single-read kernel (strips renormalised
@@ -151,12 +152,10 @@ typedef struct vd_tuning {
   int pair_split;       /* two-read items with at least this many rows per lane (6, the default, or 7)
                            run on the 12-warp-per-SM kernel (168 registers), fewer rows on the
                            16-warp kernel (128 registers); 0 = 6 */
-  int long_group;       /* VD_LONG_WARP: haplotypes per long-read item, 1..8 (0 = 8).  The item's
-                           warp runs them two at a time; the pairs after the first take each
-                           strip's lane boosts from the first pair's measured decays (the read's
-                           errors sit at the same rows against every haplotype), so fewer strips
-                           run twice.  Fewer haplotypes per item leave more items for a batch
-                           of few long reads.  VD_LONG_BLOCK items hold two haplotypes. */
+  int long_group;       /* VD_LONG_WARP: haplotypes per long-read item, 1..8 (0 = 8), run two at
+                           a time (an odd one alone).  It sets which haplotypes share a warp and
+                           the order of the work; a pair's likelihood does not depend on it.
+                           VD_LONG_BLOCK items hold two haplotypes. */
   int reserved[1];      /* must be zero */
 } vd_tuning;
 enum { VD_LONG_WARP = 0, VD_LONG_SINGLE = 1, VD_LONG_BLOCK = 2 };

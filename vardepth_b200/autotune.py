@@ -17,22 +17,15 @@ lays out the work list:
 * ``max_item_columns``  how many haplotype columns one work item streams
   (shorter items balance the tail of the persistent queue, longer ones pay
   the 31-step wavefront ramp less often);
-* ``long_mode``  how reads longer than one strip run: the warp-per-pair or
-  block-per-pair split -- a read against two haplotypes per warp with
-  per-lane power-of-two boosts (``VD_LONG_WARP``), the same items on a whole
-  CTA whose warps split each strip (``VD_LONG_BLOCK``: more parallelism per
-  pair, for batches of few long pairs), or one pair per warp in the
-  single-read kernel with exact strip renormalisation and the drift tier
-  behind it (``VD_LONG_SINGLE``);
-* ``long_group``  haplotypes per warp item of a long read: the pairs after
-  an item's first start each strip from the lane boosts the first pair
-  measured, so larger items rerun fewer strips, smaller ones leave more items
-  to balance the tail of a batch of few long reads.  It is not searched: the
-  tail it trades against depends on how many long items the whole batch
-  holds, which a sample does not show (on the mixed-length workload a 2%
-  sample preferred 4 haplotypes per item, the 20,000-region batch runs 5%
-  faster with 8).  The default (8) stays; a batch of few long reads is better
-  served by the block or single-read path, which the search does cover.
+* ``long_mode``  how reads longer than one strip run: a read against two
+  haplotypes at a time, a warp per strip with the strips of a pair side by
+  side (``VD_LONG_WARP``), on a whole CTA whose warps split each tall strip in
+  lockstep (``VD_LONG_BLOCK``), or one pair per warp in the single-read kernel
+  with exact strip renormalisation and the drift tier behind it
+  (``VD_LONG_SINGLE``);
+* ``long_group``  haplotypes per item of a long read: which of them share a
+  warp, and the order of the work.  It is not searched: every strip is its
+  own task, so the grouping hardly matters.
 
 ``autotune`` times candidate settings with resident plans (CUDA events around
 the captured tier graph) on a seeded region sample of the caller's batch,

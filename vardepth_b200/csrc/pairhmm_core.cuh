@@ -126,6 +126,13 @@ struct QueueView {
   int* error_flag;            // set when the spill list overflows
   int static_order;           // 1: warp w takes items w, w + W, w + 2W ... (W = warps in the grid)
   unsigned long long* strip_runs;  // long-read kernel, nullable: [0] runs of strips, [1] strips
+  // long-read kernel: tasks (strips of pairs), the number of each item's first
+  // task, one word per task (pairhmm_long.cuh), and where a boundary buffer's
+  // block exponents start (in 16-byte records)
+  long long long_tasks;
+  const int64_t* long_off;
+  unsigned long long* long_words;
+  long long long_exp_off;
 };
 
 }  // namespace vd

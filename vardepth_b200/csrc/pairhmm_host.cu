@@ -320,6 +320,15 @@ int rows_per_lane(int n, int long_R = kMaxR) {
   return std::min(kMaxR, std::max(1, (n + kWarp - 1) / kWarp));
 }
 
+// Rows per lane of a long read: as many strips as the strip height asks for,
+// of the fewest rows that hold the read (a 300-base read takes two strips of
+// 160 rows rather than of 256).  The block kernel and 128-row strips keep theirs.
+int long_rows(int n, const BuildOpts& bo) {
+  if (bo.long_block || bo.long_R != kMaxR) return bo.long_R;
+  const int strips = (n + kStripRows - 1) / kStripRows;
+  return (n + kWarp * strips - 1) / (kWarp * strips);
+}
+
 BuildOpts build_opts(const vd_engine* e) {
   BuildOpts bo;
   bo.long_R = e->tuning.long_read_rows / kWarp;
@@ -362,9 +371,16 @@ struct HostChunk {
   int64_t n_paired_wide = 0;       // the first of them, with pair_split..8 rows per lane
   int pair_split = 6;              // rows per lane from which two-read items run at 12 warps per SM
   int64_t n_long = 0;              // the items after them: long reads, two haplotypes per item
-  int long_R = kMaxR;              // rows per lane of those
-  bool long_block = false;         // and their kernel: block per item (else warp per item)
+  int long_R = kMaxR;              // rows per lane of those, at most
+  bool long_block = false;         // and their kernel: block per item (else a warp per strip of a pair)
+  bool strip_singles = false;      // single-read items with reads longer than a strip beside them
+  std::vector<int64_t> long_off;   // first task (strip of a pair) of each, and the total (not block)
 };
+
+// Records (16 bytes) of one of the two boundary buffers a warp slot of the
+// long-read kernel owns: a record per column, then two exponents (8 bytes) for
+// every 8 columns, in whole windows of 32.
+int64_t long_buffer_records(int64_t max_hap) { return max_hap + 1 + 2 * (max_hap / kWarp + 3); }
 
 // The robust tier runs on a small grid: it only sees pairs the FP64 wavefront
 // could not resolve, and its strip scratch then stays small.
@@ -589,12 +605,13 @@ void build_region_chunk(const vd_batch* b, int64_t g0, int64_t g1, const TableSe
                               c.hap_share.data() + (h_lo - c.ha));
     // a long read (FP32 semiglobal, one-sided emission) against its region's
     // non-empty haplotypes: runs of up to long_group neighbours per item, in
-    // both schedules (the haplotypes after an item's first pair take their
-    // boosts from it, so the grouping is part of the result)
+    // both schedules (two of an item share a warp)
     auto emit_long = [&](int64_t r) {
       const int32_t code = c.read_code[r - c.ra];
       const int n = (int)(c.read_off[r - c.ra + 1] - c.read_off[r - c.ra]);
-      const int64_t rows = (int64_t)kWarp * bo.long_R * ((n + kWarp * bo.long_R - 1) / (kWarp * bo.long_R));
+      const int strips = (n + kWarp * bo.long_R - 1) / (kWarp * bo.long_R);
+      const int R = long_rows(n, bo);
+      const int64_t rows = (int64_t)kWarp * R * strips;
       auto len = [&](int64_t h) { return (int)(b->hap_off[h + 1] - b->hap_off[h]); };
       for (int64_t h = h_lo; h < h_hi;) {
         if (len(h) <= 0) { ++h; continue; }
@@ -611,7 +628,7 @@ void build_region_chunk(const vd_batch* b, int64_t g0, int64_t g1, const TableSe
         w.nhap = k;
         w.hap_begin = h - c.ha;
         w.out_begin = region_out + (r - r_lo) * nh + (h - h_lo);
-        w.code = (code & ~15) | bo.long_R | kLongBit;
+        w.code = (code & ~15) | R | kLongBit;
         w.read2 = -1;
         w.out2_begin = 0;
         items.push_back(w);
@@ -722,6 +739,19 @@ void build_region_chunk(const vd_batch* b, int64_t g0, int64_t g1, const TableSe
   c.n_paired_wide = (int64_t)(wide - c.items.begin());
   auto lend = std::stable_partition(mid, c.items.end(), [](const WorkItem& w) { return code_long(w.code); });
   c.n_long = (int64_t)(lend - mid);
+  c.strip_singles = c.n_long > 0 && std::any_of(lend, c.items.end(), [](const WorkItem& w) { return (w.code & 512) != 0; });
+  c.long_off.clear();
+  if (c.n_long > 0 && !c.long_block) {
+    c.long_off.resize((size_t)c.n_long + 1);
+    int64_t tasks = 0;
+    for (int64_t k = 0; k < c.n_long; ++k) {
+      const WorkItem& w = c.items[(size_t)(c.n_paired + k)];
+      const int64_t n = c.read_off[w.read + 1] - c.read_off[w.read], rows = (int64_t)kWarp * code_R(w.code);
+      c.long_off[(size_t)k] = tasks;
+      tasks += (w.nhap + 1) / 2 * ((n + rows - 1) / rows);
+    }
+    c.long_off[(size_t)c.n_long] = tasks;
+  }
 }
 
 // Pair form: pairs grouped by read (counting sort), each read's haplotypes as
@@ -802,13 +832,14 @@ void build_pair_chunk(const vd_batch* b, const PairGroups& pg, int64_t ra, int64
 
 // Device bytes a chunk needs (inputs, lists, outputs, rescue lists, scratch).
 struct Layout {
-  size_t o_rb, o_rq, o_roff, o_rcode, o_hb, o_hoff, o_hsel, o_osel, o_hord, o_hshare, o_items, o_out, o_sp1,
-      o_sp2, o_cnt, o_scratch, total;
+  size_t o_rb, o_rq, o_roff, o_rcode, o_hb, o_hoff, o_hsel, o_osel, o_hord, o_hshare, o_items, o_loff, o_out, o_sp1,
+      o_sp2, o_cnt, o_lword, o_scratch, o_long, total;
   int64_t scratch_stride;  // double2 records per warp slot
+  int64_t long_stride;     // the same of the long-read kernels (two boundary buffers)
   int64_t warps;
 };
 
-Layout layout_for(const HostChunk& c, const vd_batch* b, int64_t warps) {
+Layout layout_for(const HostChunk& c, const vd_batch* b, int64_t warps, int64_t long_warps) {
   Layout L{};
   size_t off = 0;
   auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + std::max<size_t>(bytes, 1), 256); return o; };
@@ -825,14 +856,23 @@ Layout layout_for(const HostChunk& c, const vd_batch* b, int64_t warps) {
   L.o_hord = take(c.hap_order.size() * sizeof(int32_t));
   L.o_hshare = take(c.hap_share.size() * sizeof(int32_t));
   L.o_items = take(c.items.size() * sizeof(WorkItem));
+  L.o_loff = take(c.long_off.size() * sizeof(int64_t));
   L.o_out = take((size_t)c.n_out * sizeof(double));
   L.o_sp1 = take((size_t)std::max<int64_t>(1, c.pairs_scored) * sizeof(RescueEntry));
   L.o_sp2 = take((size_t)std::max<int64_t>(1, c.pairs_scored) * sizeof(RescueEntry));
   L.o_cnt = take(16 * sizeof(unsigned long long));
-  // the long-read kernel keeps two boundary buffers per warp slot
-  L.scratch_stride = c.any_long ? (int64_t)(c.max_hap + 1) * (c.n_long > 0 ? 2 : 1) : 0;
+  // one word per task of the long-read kernel, right behind the counters (cleared with them)
+  L.o_lword = take(c.long_off.empty() ? 0 : (size_t)c.long_off.back() * sizeof(unsigned long long));
+  // one boundary per warp slot of the tiers.  The long-read kernels use the same
+  // bytes as two buffers per warp: the rescue tiers start when they are done; only
+  // the single-read kernel beside them, when it strip-mines reads too (long
+  // reads with Phred 0 or 1 bases), needs its own.
+  L.scratch_stride = c.any_long ? (int64_t)c.max_hap + 1 : 0;
+  L.long_stride = c.n_long > 0 ? 2 * long_buffer_records(c.max_hap) : 0;
   L.warps = c.any_strip ? warps : std::min<int64_t>(warps, (int64_t)kRobustBlocks * kWarpsPerBlock);
-  L.o_scratch = take((size_t)std::max<int64_t>(1, L.scratch_stride) * warps * sizeof(double2));
+  const int64_t own = std::max<int64_t>(1, L.scratch_stride) * warps, shared = L.long_stride * long_warps;
+  L.o_scratch = take((size_t)(c.strip_singles ? own : std::max(own, shared)) * sizeof(double2));
+  L.o_long = c.strip_singles ? take((size_t)shared * sizeof(double2)) : L.o_scratch;
   L.total = off;
   (void)b;
   return L;
@@ -950,6 +990,7 @@ int upload_chunk(vd_plan* pl, const vd_batch* b, int64_t* h2d) {
   if ((rc = put(pl->L.o_hord, c.hap_order.data(), c.hap_order.size() * sizeof(int32_t)))) return rc;
   if ((rc = put(pl->L.o_hshare, c.hap_share.data(), c.hap_share.size() * sizeof(int32_t)))) return rc;
   if ((rc = put(pl->L.o_items, c.items.data(), c.items.size() * sizeof(WorkItem)))) return rc;
+  if ((rc = put(pl->L.o_loff, c.long_off.data(), c.long_off.size() * sizeof(int64_t)))) return rc;
   if (c.n_out > 0) {
     fill_kernel<<<(int)std::min<int64_t>(4096, (c.n_out + 255) / 256), 256, 0, pl->stream>>>(
         (double*)(d + pl->L.o_out), c.n_out, -HUGE_VAL);
@@ -976,7 +1017,8 @@ int enqueue_tiers(vd_plan* pl, int* launches, bool capturing = false) {
   // cnt[6..7] heads of the two-read kernels, cnt[8] spill count of the FP64
   // tier, cnt[9] head of the drift tier (FP32 semiglobal only), cnt[10]
   // head of the long-read kernel, cnt[11..12] its runs of strips and strips
-  VD_CUDA(cudaMemsetAsync(cnt, 0, 16 * sizeof(unsigned long long), pl->stream));
+  const int64_t long_tasks = pl->chunk.long_off.empty() ? 0 : pl->chunk.long_off.back();
+  VD_CUDA(cudaMemsetAsync(cnt, 0, L.o_lword - L.o_cnt + (size_t)long_tasks * sizeof(unsigned long long), pl->stream));
   VD_CUDA(cudaEventRecordWithFlags(pl->ev_begin, pl->stream, evflags));
   const BatchView bv = batch_view(pl);
   // device tables by address; the scalars by value from the host copy
@@ -1003,17 +1045,22 @@ int enqueue_tiers(vd_plan* pl, int* launches, bool capturing = false) {
     const int64_t nl = pl->chunk.n_long;
     q.static_order = pl->params.schedule == VD_SCHEDULE_PLAIN ? 1 : 0;
     if (nl > 0) {
-      // long reads, up to kLongGroupMax haplotypes per warp item, launched
-      // first on the side stream: the kernels below take the SMs its blocks
-      // leave as its queue runs dry, so they fill its tail; its failures join
-      // the spill list
+      // long reads, a warp per strip of a pair of haplotypes, launched first on
+      // the side stream: the kernels below take the SMs its blocks leave as its
+      // queue runs dry, so they fill its tail; its failures join the spill list
       VD_CUDA(cudaEventRecord(pl->ev_fork, pl->stream));
       VD_CUDA(cudaStreamWaitEvent(pl->side, pl->ev_fork, 0));
       QueueView ql = q;
       ql.items = (const WorkItem*)(d + L.o_items) + np;
       ql.n_items = nl;
       ql.head = cnt + 10;
+      ql.scratch = d + L.o_long;
+      ql.scratch_stride = L.long_stride;
       ql.strip_runs = cnt + 11;  // cnt[11] runs of strips, cnt[12] strips
+      ql.long_tasks = long_tasks;
+      ql.long_off = (const int64_t*)(d + L.o_loff);
+      ql.long_words = (unsigned long long*)(d + L.o_lword);
+      ql.long_exp_off = pl->chunk.max_hap + 1;
       const int R = pl->chunk.long_R;
       const bool blk = pl->chunk.long_block;
       err = launch_long_f32(R, blk, bv, ql, &dt->f32, ht->s32d, e->grid_long[blk ? 1 : 0][R == 8 ? 1 : 0], pl->side);
@@ -1124,6 +1171,7 @@ int enqueue_counter_read(vd_plan* pl, unsigned long long* host) {
 // recomputed in the FP64 wavefront (r1) and in FP64 32-row strips (r2)
 int check_counters(const vd_plan* pl, const unsigned long long* h, int64_t* r0, int64_t* r1, int64_t* r2,
                    int64_t* runs = nullptr, int64_t* strips = nullptr) {
+  if ((int)h[5] == 2) return fail(VD_ECUDA, "a long-read strip waited too long for the one above it");
   if (h[5]) return fail(VD_EOVERFLOW, "rescue list overflow");
   if (runs) *runs = (int64_t)h[11];
   if (strips) *strips = (int64_t)h[12];
@@ -1185,6 +1233,11 @@ int64_t max_grid_warps(const vd_engine* e) {
   int g = 0;
   for (int f = 0; f < 2; ++f) for (int a = 0; a < 2; ++a) g = std::max(g, e->grid[f][a]);
   return (int64_t)g * kWarpsPerBlock;
+}
+
+// warps of the kernel a chunk's long reads run on
+int64_t long_warps(const vd_engine* e, const HostChunk& c) {
+  return (int64_t)e->grid_long[c.long_block ? 1 : 0][c.long_R == kMaxR ? 1 : 0] * kWarpsPerBlock;
 }
 
 std::mutex g_default_mu;
@@ -1468,8 +1521,11 @@ int vd_forward(vd_engine* e, const vd_batch* b, const vd_params* p, double* out,
   for (int64_t h = 0; h < b->n_haps; ++h) max_hap = std::max<int64_t>(max_hap, b->hap_off[h + 1] - b->hap_off[h]);
   for (int64_t r = 0; r < b->n_reads; ++r) max_read = std::max<int64_t>(max_read, b->read_off[r + 1] - b->read_off[r]);
   const int64_t scratch_warps = max_read + p->anchored > kStripRows ? warps : std::min<int64_t>(warps, (int64_t)kRobustBlocks * kWarpsPerBlock);
-  // (two boundary buffers per warp slot when the long-read kernel runs)
-  fixed += (max_hap + 1) * scratch_warps * (int64_t)sizeof(double2) * (max_read > kStripRows ? 2 : 1) + 64 * 1024;
+  // (two boundary buffers per warp of the long-read kernel where it runs)
+  const int64_t long_w = (int64_t)e->grid_long[lbo.long_block ? 1 : 0][lbo.long_R == kMaxR ? 1 : 0] * kWarpsPerBlock;
+  fixed += std::max((max_hap + 1) * scratch_warps, max_read > kStripRows ? 2 * long_buffer_records(max_hap) * long_w : 0) *
+               (int64_t)sizeof(double2) +
+           64 * 1024;
   const int64_t budget = (int64_t)e->budget;
 
   // results of the chunk in a slot, once its stream has completed
@@ -1531,7 +1587,7 @@ int vd_forward(vd_engine* e, const vd_batch* b, const vd_params* p, double* out,
     else build_region_chunk(b, u, u_end, e->htab, offsets, p->anchored != 0, p->precision == VD_PRECISION_MIXED,
                             pl.chunk, plain, bo);
     HostChunk& c = pl.chunk;
-    pl.L = layout_for(c, b, warps);
+    pl.L = layout_for(c, b, warps, long_warps(e, c));
     s.host_ms += now_ms() - th;
     if ((rc = sl.arena.reserve(pl.L.total))) return rc;
     pl.base = (char*)sl.arena.p;
@@ -1604,7 +1660,7 @@ int vd_plan_create(vd_engine* e, const vd_batch* b, const vd_params* p, vd_plan*
     build_region_chunk(b, 0, b->n_regions, e->htab, offsets, p->anchored != 0, p->precision == VD_PRECISION_MIXED,
                        pl->chunk, plain, bo);
   }
-  pl->L = layout_for(pl->chunk, b, max_grid_warps(e));
+  pl->L = layout_for(pl->chunk, b, max_grid_warps(e), long_warps(e, pl->chunk));
   if ((rc = pl->own.reserve(pl->L.total))) { delete pl; return rc; }
   pl->base = (char*)pl->own.p;
   if ((rc = upload_chunk(pl, b, nullptr))) { delete pl; return rc; }

@@ -106,6 +106,9 @@ constexpr int kUnroll = 8;
 // take their own boost, measured lane by lane (a variant or a cluster of
 // errors concentrates the decay in a few rows).  What still fails goes to FP64.
 constexpr int kDriftTries = 6;
+// Reads of several strips need a gap-continuation probability of at least
+// this for FP32 to hold them (pairhmm_long.cuh); below it they go to FP64.
+constexpr float kLongMinExt = 0.0025f;
 
 // Row layout of one read (lane L, register r of strip s holds row
 // i = s*32R + L*R + r - v, 0-based):
@@ -512,6 +515,8 @@ __device__ __forceinline__ void process_item(const BatchView& bv, const QueueVie
 #pragma unroll
         for (int o = 16; o; o >>= 1) E += __shfl_xor_sync(FULL, E, o);
       }
+    } else if (sc.x < (T)kLongMinExt) {
+      ok = false;
     } else if constexpr (R == kMaxR || R == 4 || R == 2 || R == 1) {
       int Bs = SR;  // first guess: one bit per row (the spilled reads lost more than 160 per strip)
       for (int strip = 0; ok && strip < nstrips; ++strip) {

@@ -1,54 +1,77 @@
-// Long reads (more rows than one 256-row strip), FP32, semiglobal: one warp
-// runs one read against up to kLongGroupMax haplotypes of its region, TWO at
-// a time.
+// Long reads (more rows than one strip), FP32, semiglobal: a read against TWO
+// haplotypes of its region at a time, strip by strip, the strips of a pair
+// running side by side on different warps of the GPU.
 //
 // The read's rows are packed as float2 over the two haplotypes of a pair (x:
 // the first, y: the second), so every FMA serves both (fma.rn.f32x2) and the
-// read's per-row constants, its strip count and its strip bookkeeping are
-// shared: the halves always have the same number of strips, which two reads
-// of different lengths would not.  A region's haplotypes differ by a few
-// small edits, so their lengths nearly agree and the shorter one idles for a
-// few columns at most.
+// read's per-row constants and its strip count are shared: the halves always
+// have the same number of strips, which two reads of different lengths would
+// not.  A region's haplotypes differ by a few small edits, so their lengths
+// nearly agree and the shorter one idles for a few columns at most.
+//
+// Tasks.  A strip of a pair is one task; an item (a read against up to
+// kLongGroupMax haplotypes) holds its pairs' strips in order, and warps pull
+// tasks from one counter.  Strip s+1 follows strip s at a distance of about
+// three windows of 32 columns, reading the boundary rows s has published so
+// far, so a pair takes about one strip's time plus that distance per strip
+// instead of its strips one after another.  Every wait is for a task with a
+// smaller number, which some resident warp has already pulled, so the lowest
+// unfinished task can always go on; the waits are bounded all the same.
 //
 // Range.  An error-rich read (8% errors at reported Q30) loses about one bit
-// per row along its best path, far more over a 256-row strip than FP32 holds,
-// so lane L scales everything it takes from above by 2^k_L.  A boost on a
-// lane's inputs scales the lane's rows and everything below by an exact power
-// of two, so the rows keep the one-sided emission (a match costs no multiply)
-// and the boosts are undone exactly in the final exponent.  The first pair of
-// an item spreads each strip's predicted decay (the read's mean rate so far
-// times the strip's rows) evenly over the lanes; a strip whose bottom leaves
-// 2^-60 .. 2^60, or a lane whose bottom-row maximum leaves 2^-90 .. 2^90, is
-// run again with each lane's measured decay (its input boundary is kept: the
-// warp's slot holds two boundary buffers, one read and one written).  The
-// pairs after the first start each strip from the first pair's measured lane
-// decays, since the read's errors sit at the same rows against every
-// haplotype.  The first strip starts from 2^60.  A strip's boundary is stored
-// as computed and brought to 2^0 by an exact power of two as the next strip
-// loads it.  A pair still out of range after kLongTries runs of a strip, or
-// decaying faster than kLongMaxRate bits per row, goes to the drift and FP64
-// tiers.
+// per row along its best path, far more over a strip than FP32 holds, and
+// along a row the cells away from the path lie thousands of binary orders
+// lower.  So every lane keeps its rows' state scaled by its own power of two
+// 2^e, chosen anew every 16 steps: a value never grows along a path, so what a
+// lane can reach in the next 16 steps is bounded by the state of its own rows
+// and of the lanes (and the boundary) above it, and e puts that bound at 2^100.
+// The factor between a lane and the one above is folded into the lane's row 0,
+// so the step itself carries no scaling; all factors are exact powers of two,
+// undone in the exponent of the final sum.  What falls below 2^-126 lies more
+// than 200 binary orders below the best cell near it.
 //
-// Every choice above depends on the item's own data (a first pair's boosts on
-// that pair alone, per half; a re-run caused by the other half recomputes this
-// half's strip bit for bit; the later pairs' on the first pair's
-// measurements), and the final log is taken as ln f + (e - E) ln 2 with the
-// sum z = f 2^e, so the bits do not depend on which powers of two the boosts
-// took.  The plain schedule forms the same items and gives the same bits.
+// Nothing depends on which warp runs a task or when: a pair's result is a
+// function of the read and its two haplotypes.  The final log is taken as
+// ln f + (e + E) ln 2 with the sum z = f 2^e, so the bits do not depend on the
+// powers of two either.  The plain schedule forms the same pairs and gives the
+// same bits.
+//
+// What bounds it: alone, the chain of a strip's steps; in a full batch, issue
+// slots and latency at 12 warps per SM (115 warp instructions a step for 256 x 2
+// cells, 72 of them the rows; a quarter of the stalls are boundary words from
+// L2).  Measured against a warp per item (its strips one after another, re-run
+// with measured boosts when they left the FP32 range: 1.11 runs per strip): 30
+// reads of 1-10 kb, 375 pairs, 388 -> 9.2 ms; 400 mixed-length regions 390 -> 28 ms;
+// 16,000 of them (2.5e12 cells) 804 -> 782 ms, their long reads alone 557 -> 486 ms
+// (2,586 GCUPS).  Exponents every 16 steps cost 12% against every 32, which a
+// 40-base insertion run would defeat; letting a waiting strip fall 1 or 3 blocks
+// further back, to meet the one above less often, cost 3% and 8%.
+//
+// VD_LONG_BLOCK (below) runs an item on a block: the CTA's warps split each
+// tall strip in lockstep, with one boost per warp and strip.
 #pragma once
 #include "pairhmm_kernel.cuh"
 
 namespace vd {
 
-constexpr int kLongTries = 6;       // runs of one strip before a half gives up
-// A strip bottom must end in 2^-60 .. 2^60: the cells that carry the mass lie
-// within a few dozen binary orders below the bottom's maximum, and they must
-// stay far above 2^-126, where the packed f32x2 arithmetic loses them (with
-// bottoms allowed down to 2^-100 the error reached 8e-4 log10 on 8%-error
-// 7 kb reads, down to 2^-120 0.1; at 2^-60 it stays at the FP32 rounding level)
+// A pair that has decayed by more than this many bits over its read's first
+// `rows` rows goes to the drift and FP64 tiers: an error-rich read takes about one
+// bit per row; a random read against a random haplotype takes four to five, and
+// there alignment families that trade places across rows lie hundreds of bits
+// apart (restated on the CPU against the oracle: exact to FP32 rounding below
+// 4.0 bits per row, off by up to 0.2 log10 at 4.0 to 4.4).
+__host__ __device__ constexpr int long_max_bits(int rows) { return rows * 15 / 4; }
+constexpr int kLongTop = 100;             // a lane's bound for the coming steps, binary orders
+constexpr int kLongNone = -(1 << 28);     // exponent of "nothing there"
+constexpr long long kLongSpins = 1ll << 25;  // polls of one wait before it gives up (tens of seconds)
+
+// VD_LONG_BLOCK: runs of one tall strip before a half gives up, the window its
+// warps' bottoms must end in (cells a few dozen binary orders below a bottom's
+// maximum carry mass and must stay above 2^-126), and the first strip's input.
+constexpr int kLongTries = 6;
 constexpr int kLongFloor = -60;
 constexpr int kLongCeil = 60;
-constexpr int kLongStart = 60;      // the first strip's input, 2^60 (binary orders)
+constexpr int kLongStart = 60;
 
 template <int R>
 struct LongRows {
@@ -109,67 +132,80 @@ __device__ __forceinline__ int long_exponent(double v) {
   return (v != v || v >= HUGE_VAL) ? 1024 : (v > 0.0 ? ilogb(v) : -1024);
 }
 
-// One half's lane boosts after a run of a strip that left the window.  Lane
-// L measured the maximum of its bottom row (exponent lg_L, +-1024 for inf or
-// zero); with its input at 2^lg_{L-1} (lane 0: the strip's input, 2^in0) and
-// boost k_L, its rows decayed by d_L = k_L + lg_{L-1} - lg_L bits, and the
-// boost d_L (lane 0: d_0 - in0) brings its bottom to 2^0 wherever in the
-// strip the read's errors sit.  The first lane whose bottom under- or
-// overflowed moves by the bound that shows (a nonzero float lies above
-// 2^-149, a finite one below 2^128), and the lanes below it, whose inputs
-// are unknown, take the mean rate of the lanes above.  Shares stay within
-// -96 .. 120 bits, where 2^k times every row factor is a normal float.
-__device__ __forceinline__ int relane(const int kl, const float lm, const int used, const int lrows, const int in0,
-                                      const int lane) {
-  constexpr unsigned FULL = 0xffffffffu;
-  const int lg = lane < used ? long_exponent(lm) : 0;
-  int in = __shfl_up_sync(FULL, lg, 1);
-  if (lane == 0) in = in0;
-  const int tgt = lane == 0 ? in0 : 0;  // the input the next run's lane sees
-  const bool measured = lg > -1024 && lg < 1024;
-  const unsigned bad = __ballot_sync(FULL, lane < used && !measured);
-  const int first_bad = bad ? __ffs(bad) - 1 : kWarp;
-  const bool valid = lane < used && lane < first_bad;
-  const int d = valid ? kl + in - lg : 0;
-  int sum_d = d, sum_r = valid ? lrows : 0;
-#pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    sum_d += __shfl_xor_sync(FULL, sum_d, o);
-    sum_r += __shfl_xor_sync(FULL, sum_r, o);
-  }
-  if (lane >= used) return 0;
-  int k = kl;
-  if (valid) {
-    k = d - tgt;
-  } else {
-    if (sum_r > 0) k = (int)((long long)sum_d * lrows / sum_r) - tgt;
-    if (lane == first_bad) k = lg == -1024 ? max(k, kl + in + 149 - tgt) : min(k, kl + in - 128 - tgt);
-  }
-  return max(-96, min(120, k));
+
+// Steps between two choices of the lanes' exponents.  A lane's bound counts
+// the lanes that a path can come down from by matches alone (span / R + 1)
+// at their full value, so a path that runs down a column by insertions
+// instead lies up to (span + 2 R) log2(4/x) bits and a gap opening below it: at
+// x = 0.1 190 bits for 16 steps, of the 226 between the bound and 2^-126;
+// smaller x needs 8.  Below kLongMinExt (pairhmm_kernel.cuh) a read that hangs
+// off the haplotype's end has no cheap way down, its best path lies hundreds of
+// bits below one that ends there, and the pair goes to the FP64 tier (restated
+// on the CPU against the oracle over reads hanging off by up to 40 bases: exact
+// to FP32 rounding from x = 0.003 up, off by up to 1e-1 log10 at 0.001).
+constexpr int kLongSpan = 16, kLongSpanShort = 8;
+
+__device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_release(unsigned long long* p, unsigned long long v) {
+  asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-// Strips of a read whose per-lane decays the first pair of an item records
-// (longer reads predict the rest from the mean rate), and the window a lane's
-// bottom-row maximum must end in for a run to be kept.
-constexpr int kLongProfStrips = 80;
-// Boost bits per row a strip may take (an error-rich read at 8% errors and
-// reported Q30 takes about one; a random read against a random haplotype
-// four to five)
-constexpr int kLongMaxRate = 4;
-constexpr int kLongLaneFloor = -90;
-constexpr int kLongLaneCeil = 90;
+// A task's word: boundary blocks published so far (all of them: the task is
+// done), which halves left the range, and the buffer its boundary is in.
+__device__ __forceinline__ int task_blocks(unsigned long long v) { return (int)(v & 0x3fffffffull); }
+__device__ __forceinline__ unsigned task_fail(unsigned long long v) { return (unsigned)(v >> 30) & 3u; }
+__device__ __forceinline__ int task_buffer(unsigned long long v) { return (int)(v >> 32); }
 
-// One work item: read w.read against haplotypes hap_begin .. hap_begin +
-// nhap - 1 (nhap <= kLongGroupMax), two at a time; outputs out_begin + k.
-// `scratch` is the warp's slot: 2 * half float4 boundary records (half >= the
-// longest haplotype + 1); `ring` and `oring` 32 float4 each of shared memory
-// per warp (the boundary read, the boundary written); `prof` the warp's
-// kLongProfStrips x 32 per-lane decays.
-template <int R>
-__device__ __noinline__ void process_long(const BatchView bv, const QueueView qv, const WorkItem w,
-                                          const Tables<float>* __restrict__ tb, const Scalars<float> sc,
-                                          const int lane, float4* __restrict__ scratch, float4* __restrict__ ring,
-                                          float4* __restrict__ oring, short* __restrict__ prof) {
+// Waits until the task behind `p` has published `need` blocks; returns its
+// word.  Every lane polls (one broadcast load).  After kLongSpins polls, or
+// once another wait has given up, the error flag is set and ok is false.
+__device__ __forceinline__ unsigned long long wait_task(const unsigned long long* p, int need, int* error_flag,
+                                                        bool& ok) {
+  unsigned long long v = ld_acquire(p);
+  for (long long spin = 0; task_blocks(v) < need; ++spin) {
+    if (spin >= kLongSpins || ((spin & 1023) == 1023 && *(volatile int*)error_flag != 0)) {
+      atomicExch(error_flag, 2);
+      ok = false;
+      break;
+    }
+    __nanosleep(64);
+    v = ld_acquire(p);
+  }
+  ok = __all_sync(0xffffffffu, ok);
+  return v;
+}
+
+// exponent of a non-negative float, kLongNone below the normal range
+__device__ __forceinline__ int state_exponent(float v) {
+  const int e = (int)((unsigned)__float_as_int(v) >> 23);
+  return e == 0 ? kLongNone : e - 127;
+}
+__device__ __forceinline__ float normal_or_0(float v) { return v < 1.17549435e-38f ? 0.f : v; }
+// v 2^k for any k: two exact factors (0 or inf past the range)
+__device__ __forceinline__ float scale2(float v, int k) {
+  k = max(-252, min(252, k));
+  const int a = max(-126, min(126, k));
+  return (v * pow2T(a, 0.f)) * pow2T(k - a, 0.f);
+}
+
+// One task: strip `strip` of item w's pair g (haplotypes g, g+1 of the item).
+// `task` is its number; `half` the records of one boundary buffer (the block
+// exponents follow at record exp_off); `bufs` the first buffer, `mine` the
+// buffer this task writes.  `ring` and `oring` (32 float4 each) and `oexp` (4
+// int2) are the warp's shared memory: the boundary read, the boundary written
+// and lane 31's exponents of its four groups of 8 columns.  Returns
+// false when a wait gave up.
+template <int R, int SPAN>
+__device__ __forceinline__ bool long_task(const BatchView& bv, const QueueView& qv, const WorkItem& w, const int g,
+                                          const int strip, const int nstrips, const long long task,
+                                          const Tables<float>* __restrict__ tb, const Scalars<float>& sc,
+                                          const int lane, float4* const bufs, const long long half, const int mine,
+                                          float4* __restrict__ ring, float4* __restrict__ oring,
+                                          int2* __restrict__ oexp) {
   constexpr unsigned FULL = 0xffffffffu;
   constexpr double kLn2 = 0.6931471805599453094;
   constexpr int SR = kWarp * R;
@@ -177,368 +213,439 @@ __device__ __noinline__ void process_long(const BatchView bv, const QueueView qv
   const int n = (int)(bv.read_off[w.read + 1] - roff);
   const uint8_t* __restrict__ rbase = bv.read_bases + roff;
   const uint8_t* __restrict__ rqual = bv.read_quals + roff;
-  const int nstrips = (n + SR - 1) / SR;
-  const long long half = qv.scratch_stride / 2;
+  const bool two = g + 1 < w.nhap;
+  const int64_t h1 = w.hap_begin + g, h2 = two ? h1 + 1 : h1;
+  const int64_t ho1 = bv.hap_off[h1], ho2 = bv.hap_off[h2];
+  const int m1 = (int)(bv.hap_off[h1 + 1] - ho1), m2 = (int)(bv.hap_off[h2 + 1] - ho2);
+  const uint8_t* __restrict__ hp1 = bv.hap_bases + ho1 - 1;  // hp[j] = base of column j >= 1
+  const uint8_t* __restrict__ hp2 = bv.hap_bases + ho2 - 1;
+  const int M = max(m1, m2);
+  const bool first = strip == 0, last = strip == nstrips - 1;
+  if (sc.x < kLongMinExt) {  // the whole pair to the next tiers
+    if (last && lane < (two ? 2 : 1)) {
+      const int64_t o = w.out_begin + g + lane;
+      bv.out[o] = __longlong_as_double(0x7ff8000000000000LL);
+      spill_pair<float>(qv, w.read, h1 + lane, o);
+    }
+    if (lane == 0) {
+      st_release(qv.long_words + task, 0x3fffffffull);
+      if (qv.strip_runs != nullptr) {
+        atomicAdd(qv.strip_runs, 1ull);
+        atomicAdd(qv.strip_runs + 1, 1ull);
+      }
+    }
+    return true;
+  }
+  // windows of 32 steps; lane 31 finishes columns 32 (w-1) + 1 .. 32 w in window w (block w)
+  const int nwin = (M + kWarp - 1) / kWarp + 1;
+  unsigned long long* const word = qv.long_words + task;
+  const unsigned long long* const above = word - 1;
+  int* const err = qv.error_flag;
+  bool ok = true;
 
-  double lnN = 0.0;
-  for (int i = lane; i < n; i += kWarp) lnN += tb->lnN[rqual[i]];
+  LongRows<R> rw;
+  const int i0 = strip * SR;
 #pragma unroll
-  for (int o = 16; o; o >>= 1) lnN += __shfl_xor_sync(FULL, lnN, o);
-  const float A = tb->A[rqual[n - 1]];
-  const float2 k2 = make_float2(sc.k2, sc.k2), x = make_float2(sc.x, sc.x);
-  const float c0 = sc.c;
+  for (int r = 0; r < R; ++r) {
+    const int i = i0 + lane * R + r;
+    if (i < n) {
+      const unsigned q = rqual[i];
+      rw.rb[r] = rbase[i];
+      rw.miss[r] = tb->miss[q];
+      const float K = tb->K[q], X = (i == n - 1) ? tb->A[q] : tb->X[q];
+      rw.K[r] = make_float2(K, K);
+      rw.X[r] = make_float2(X, X);
+    } else {  // past the read: pass u down the column
+      rw.rb[r] = kNeverBase;
+      rw.miss[r] = 0.f;
+      rw.K[r] = make_float2(0.f, 0.f);
+      rw.X[r] = make_float2(1.f, 1.f);
+    }
+    rw.W[r] = make_float2(0.f, 0.f);
+    rw.s[r] = make_float2(0.f, 0.f);
+  }
+  const float K0 = rw.K[0].x, X0 = rw.X[0].x;  // row 0's own factors (those in rw carry the lane factor)
+  // bits a path loses when it crosses this lane by insertions, one run of them
+  // (X per row) or single ones (K), summed over the lanes down to this one (the lanes past the read lose nothing, and no path
+  // to a lane of the read crosses its last one)
+  const int used = (min(SR, n - i0) + R - 1) / R;  // lanes holding read rows
+  constexpr int reach = SPAN / R + 1;
+  int cross = 0, slack = 0, row_bits = 30;
+  {
+    float b = 0.f;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const float c = -log2f(fmaxf(rw.X[r].x, rw.K[r].x));
+      b += c;
+      if (i0 + lane * R + r < n) row_bits = min(row_bits, (int)floorf(fminf(30.f, c - 0.01f)));
+    }
+    row_bits = max(0, __reduce_min_sync(FULL, row_bits));  // per row, at least
+    // (at most 96, so that neighbours' exponents differ by less than a float's range)
+    const int bits = max(0, (int)floorf(fminf(96.f, b - 0.01f)));
+    // a path may take its matches in whichever lanes cost most by insertions
+    slack = reach * max(0, __reduce_max_sync(FULL, lane < used - 1 ? bits : 0) -
+                               __reduce_min_sync(FULL, lane < used - 1 ? bits : 1 << 20));
+    cross = lane < used - 1 ? bits : 0;
+#pragma unroll
+    for (int o = 1; o < kWarp; o <<= 1) {
+      const int v = __shfl_up_sync(FULL, cross, o);
+      if (lane >= o) cross += v;
+    }
+  }
 
-  // the item's first pair records each strip's per-lane decays (of its first
-  // half while that is in play, else its second); the pairs after it start a
-  // recorded strip from them and the rest from the mean rate
-  int prof_len = 0;
-  // every lane holding read rows ended its bottom row in the lane window
-  auto lanes_in_window = [&](const float lm, const int used) -> bool {
-    const int lg = long_exponent(lm);
-    return __all_sync(FULL, lane >= used || (lg >= kLongLaneFloor && lg < kLongLaneCeil));
+  // boundary above: lane i of window w holds column 32 w + i, raw, with the
+  // exponents of the block it came in
+  const float4* src = nullptr;
+  const int2* src_exp = nullptr;
+  float4 nxt = make_float4(0.f, 0.f, 0.f, 0.f);
+  int2 nexp = make_int2(0, 0);
+  int published = 0;  // blocks of the strip above known to be published
+  auto load_window = [&](int wn) {
+    if (published < min(wn + 2, nwin)) {
+      const unsigned long long v = wait_task(above, min(wn + 2, nwin), err, ok);
+      published = task_blocks(v);
+      if (src == nullptr) {
+        src = bufs + (long long)task_buffer(v) * half;
+        src_exp = reinterpret_cast<const int2*>(src + qv.long_exp_off);
+      }
+    }
+    const int p = wn * kWarp + lane;
+    if (ok && p <= M) {
+      nxt = __ldcg(src + p);
+      // (denormals would count for nothing in the bound and still be scaled up)
+      nxt = make_float4(normal_or_0(nxt.x), normal_or_0(nxt.y), normal_or_0(nxt.z), normal_or_0(nxt.w));
+      nexp = __ldcg(src_exp + ((p + kWarp - 1) >> 3));
+    } else {
+      nxt = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  };
+  if (first) {
+    nxt = make_float4(sc.c, sc.c, sc.c, sc.c);  // row 0: c at every column
+  } else {
+    load_window(0);
+    if (!ok) return false;
+  }
+  float4* const dst = bufs + (long long)mine * half;
+  int2* const dst_exp = reinterpret_cast<int2*>(dst + qv.long_exp_off);
+  const unsigned long long tag = (unsigned long long)(unsigned)mine << 32;
+
+  int ex = 0, ey = 0;  // the lane's state is scaled by 2^-e
+  float2 s_top = make_float2(0.f, 0.f), u_bot = make_float2(0.f, 0.f), acc32 = make_float2(0.f, 0.f);
+  double accx = 0.0, accy = 0.0;            // row sums of the window (scale of e)
+  double totx = 0.0, toty = 0.0;            // row sums so far, times 2^-E
+  int Ex = kLongNone, Ey = kLongNone;
+  int bmx = kLongNone, bmy = kLongNone;     // exponents of the bottom row's maxima (this lane's columns)
+  const bool lane0 = lane == 0;
+
+  int in_x = kLongNone, in_y = kLongNone;  // exponents of the window's largest inputs
+  auto add_total = [&](double& acc, int e, double& tot, int& E) {
+    if (acc > 0.0) {
+      if (E == kLongNone) {
+        tot = acc;
+        E = e;
+      } else if (e > E) {
+        tot = ldexp(tot, max(-2000, E - e)) + acc;
+        E = e;
+      } else {
+        tot += ldexp(acc, max(-2000, e - E));
+      }
+    } else if (acc != acc) {
+      tot = acc;
+    }
+    acc = 0.0;
   };
 
-  for (int g = 0; g < w.nhap; g += 2) {
-    // the pair in hand
-    const bool two = g + 1 < w.nhap;
-    const int64_t h1 = w.hap_begin + g, h2 = two ? h1 + 1 : h1;
-    const int64_t ho1 = bv.hap_off[h1], ho2 = bv.hap_off[h2];
-    const int m1 = (int)(bv.hap_off[h1 + 1] - ho1), m2 = (int)(bv.hap_off[h2 + 1] - ho2);
-    const uint8_t* __restrict__ hp1 = bv.hap_bases + ho1 - 1;  // hp[j] = base of column j >= 1
-    const uint8_t* __restrict__ hp2 = bv.hap_bases + ho2 - 1;
-    const int M = max(m1, m2);
-
-    // per half: boost bits of the current strip, total exponent, still in play
-    int Bx = 0, By = 0, Ex = 0, Ey = 0;
-    // decay measured over the strips done so far (bits, rows): the next strip's
-    // boost is this mean rate times its rows.  A single strip's decay scatters
-    // by tens of bits around the read's rate (the number of errors in 256 rows),
-    // so the mean predicts the next strip about sqrt(2) times better than the
-    // last strip alone, and fewer strips run twice
-    int Dx = 0, Dy = 0, Nrows = 0;
-    bool okx = true, oky = two;
-    int inx = 0, iny = 0;        // shifts that bring the boundary above to 2^0, per half
-    int lgx = 0, lgy = 0;        // bottom exponents of the last run
-    double zx = 0.0, zy = 0.0;   // final sums (last strip, lane 31)
-    int klx = 0, kly = 0;        // this lane's share of the strip's boost, per half
-    float lmx = 0.f, lmy = 0.f;  // this lane's bottom-row maxima in the last run
-
-    // One run of strip `strip` with Bx / By boost bits; reads boundary buffer
-    // src_half, writes the other.  Sets lgx / lgy (bottom maximum or final sum).
-    auto run_strip = [&](const int strip, const bool last) {
-      const int i0 = strip * SR;
-      const int ns = min(SR, n - i0);           // read rows of the strip
-      const int lanes_used = (ns + R - 1) / R;  // lanes holding read rows
-      LongRows<R> rw;
-  #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int i = i0 + lane * R + r;
-        if (i < n) {
-          const unsigned q = rqual[i];
-          rw.rb[r] = rbase[i];
-          rw.miss[r] = tb->miss[q];
-          const float K = tb->K[q], X = (i == n - 1) ? A : tb->X[q];
-          rw.K[r] = make_float2(K, K);
-          rw.X[r] = make_float2(X, X);
-        } else {  // past the read: pass u down the column
-          rw.rb[r] = kNeverBase;
-          rw.miss[r] = 0.f;
-          rw.K[r] = make_float2(0.f, 0.f);
-          rw.X[r] = make_float2(1.f, 1.f);
-        }
-        rw.W[r] = make_float2(0.f, 0.f);
-        rw.s[r] = make_float2(0.f, 0.f);
-      }
-      // lane L's share of the boost: floor((L+1) B / lanes) - floor(L B / lanes)
-      // over the lanes holding read rows; the first strip's input starts at 2^kLongStart
-      // (|B| <= 4 ns keeps every share within +-4R, far inside the float exponent range)
-      boost_row0(rw, make_float2(pow2T(klx, 0.f), pow2T(kly, 0.f)));
-      const float cin = c0 * pow2T(kLongStart, 0.f);  // the first strip's row-0 value
-      float4* const src = scratch + (long long)(strip & 1) * half;
-      float4* const dst = scratch + (long long)((strip + 1) & 1) * half;
-      // the boundary above is stored as written (its maximum at 2^lg); it is
-      // brought to 2^0 as it is loaded, by 2^-lg per half
-      const float fsx = pow2T(inx, 0.f), fsy = pow2T(iny, 0.f);
-
-      float2 s_top = make_float2(0.f, 0.f), u_bot = make_float2(0.f, 0.f), acc32 = make_float2(0.f, 0.f);
-      double accx = 0.0, accy = 0.0;
-      float bmx = 0.f, bmy = 0.f;
-      float2 lm = make_float2(0.f, 0.f);  // this lane's bottom-row maxima
-      const bool lane0 = lane == 0;
-      // boundary records of the strip above, staged through the warp's ring:
-      // every 32 steps each lane loads one record of the next 32 columns, and
-      // at every step all lanes read the record of lane 0's column (a broadcast)
-      float4 nxt = make_float4(0.f, 0.f, 0.f, 0.f);
-      auto load_window = [&](int base) -> float4 {
-        const int p = base + lane;
-        if (strip == 0 || p > M) return make_float4(0.f, 0.f, 0.f, 0.f);
-        const float4 v = src[p];
-        return make_float4(v.x * fsx, v.y * fsx, v.z * fsy, v.w * fsy);
-      };
-      auto stage_window = [&](int t) {
-        __syncwarp();
-        ring[lane] = nxt;
-        __syncwarp();
-        nxt = load_window(t + kWarp);
-      };
-      // this strip's bottom rows: lane 31 lays each column's record into the
-      // warp's out-ring, and every 32 columns the warp writes them to the
-      // boundary buffer in one coalesced store and folds them into the maxima
-      int flushed = 0;  // columns below this are in the boundary buffer
-      auto flush_out = [&](int count) {
-        __syncwarp();
-        if (lane < count) {
-          const int p = flushed + lane;
-          const float4 rec = oring[lane];
-          dst[p] = rec;
-          if (p <= m1) bmx = fmaxf(bmx, fmaxf(rec.x, rec.y));
-          if (p <= m2) bmy = fmaxf(bmy, fmaxf(rec.z, rec.w));
-        }
-        __syncwarp();
-        flushed += count;
-      };
-      // lane 31 moves its FP32 row sums into FP64 after its columns 8r+7
-      auto flush_acc = [&]() {
-        accx += (double)acc32.x;
-        accy += (double)acc32.y;
-        acc32 = make_float2(0.f, 0.f);
-      };
-      const float2 cin2 = make_float2(cin, cin);
-      // one step; STEADY: every lane inside both haplotypes at a column >= 1
-      auto step = [&](auto steady_tag, const int t) {
-        constexpr bool STEADY = decltype(steady_tag)::value;
-        const int p = t - lane;  // this lane's column
-        // lane 0's boundary record is loaded before the shuffles, so its
-        // latency runs beside theirs rather than after them on the chain
-        // (20,000 mixed-length regions: 1,003 against 1,053 ms per step)
-        float2 in_s = cin2, in_u = cin2;
-        if (strip > 0) {
-          const float4 rec = ring[t & (kWarp - 1)];
-          in_s = make_float2(rec.x, rec.z);
-          in_u = make_float2(rec.y, rec.w);
-        }
-        float2 u_in = shfl_up2(u_bot);
-        float2 s_in = shfl_up2(rw.s[R - 1]);
-        u_in = lane0 ? in_u : u_in;
-        s_in = lane0 ? in_s : s_in;
-        bool inside = true;
-        uint32_t hbx, hby;
-        if (STEADY) {
-          hbx = hp1[p];
-          hby = hp2[p];
-        } else {
-          // column 0 has no base (kNeverBase never matches); past a haplotype's
-          // end its half reads that haplotype's last base (its columns are not used)
-          inside = p >= 0 && p <= M;
-          hbx = (inside && p > 0) ? (uint32_t)hp1[min(p, m1)] : kNeverBase;
-          hby = (inside && p > 0) ? (uint32_t)hp2[min(p, m2)] : kNeverBase;
-        }
-        column_long<R>(rw, hbx, hby, (STEADY || p > 0) ? s_top : make_float2(0.f, 0.f), u_in, k2, x, u_bot);
-        if (STEADY) {
-          lm.x = fmaxf(lm.x, u_bot.x);
-          lm.y = fmaxf(lm.y, u_bot.y);
-        } else {
-          if (inside && p <= m1) lm.x = fmaxf(lm.x, u_bot.x);
-          if (inside && p <= m2) lm.y = fmaxf(lm.y, u_bot.y);
-        }
-        if (!STEADY && p <= 0) {
-          // column 0 (and the lanes not started yet): no diagonal, no deletions
-  #pragma unroll
-          for (int r = 0; r < R; ++r) rw.W[r] = make_float2(0.f, 0.f);
-        }
-        s_top = s_in;
-        if (last) {
-          // the final row sums (lane 31's are the ones used)
-          if (STEADY) {
-            acc32 = __fadd2_rn(acc32, u_bot);
-          } else if (lane == kWarp - 1 && inside) {
-            if (p <= m1) acc32.x += u_bot.x;
-            if (p <= m2) acc32.y += u_bot.y;
-            if ((p & 7) == 7) flush_acc();
-          }
-        } else if (lane == kWarp - 1 && inside) {
-          oring[p & (kWarp - 1)] = make_float4(rw.s[R - 1].x, u_bot.x, rw.s[R - 1].y, u_bot.y);
-        }
-      };
-      // the out-ring is full when lane 31 has finished column flushed + 31
-      auto maybe_flush = [&](int t) {
-        if (!last && t - (kWarp - 1) == flushed + kWarp - 1) flush_out(kWarp);
-      };
-
-      nxt = load_window(0);
-      const int steps = M + 1 + (kWarp - 1);
-      // steady steps: every lane at a column in 1 .. min(m1, m2)
-      const int t_lo = kWarp, t_hi = min(m1, m2) + 1;
-      int t = 0;
-      for (; t < steps && (t < t_lo || (t < t_hi && (t & 7) != 0)); ++t) {
-        if ((t & (kWarp - 1)) == 0) stage_window(t);
-        step(std::false_type{}, t);
-        maybe_flush(t);
-      }
-      // blocks of 8 steps start at a multiple of 8, so lane 31's columns 8r+7
-      // fall at the block's step 6 and its out-ring fills at step 6 of every
-      // fourth block
-      for (; t + 8 <= t_hi; t += 8) {
-        if ((t & (kWarp - 1)) == 0) stage_window(t);
-  #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          step(std::true_type{}, t + u);
-          if (u == 6) {
-            if (last) flush_acc();
-            else maybe_flush(t + u);
-          }
-        }
-      }
-      for (; t < steps; ++t) {
-        if ((t & (kWarp - 1)) == 0) stage_window(t);
-        step(std::false_type{}, t);
-        maybe_flush(t);
-      }
-      if (!last && flushed <= M) flush_out(M + 1 - flushed);
-      if (!last) {
-  #pragma unroll
-        for (int o = 16; o; o >>= 1) {
-          bmx = fmaxf(bmx, __shfl_xor_sync(FULL, bmx, o));
-          bmy = fmaxf(bmy, __shfl_xor_sync(FULL, bmy, o));
-        }
-      }
-      __syncwarp();
-      if (last) {
-        zx = __shfl_sync(FULL, accx + (double)acc32.x, kWarp - 1);
-        zy = __shfl_sync(FULL, accy + (double)acc32.y, kWarp - 1);
-        lgx = long_exponent(zx);
-        lgy = long_exponent(zy);
-      } else {
-        lgx = long_exponent(bmx);
-        lgy = long_exponent(bmy);
-      }
-      lmx = lm.x;
-      lmy = lm.y;
-    };
-
-
-    // the strips, each run until both halves' bottoms are in the window
-    bool fail_x = false, fail_y = !two;
-    for (int strip = 0; strip < nstrips && (okx || oky); ++strip) {
-      const bool last = strip == nstrips - 1;
-      const int ns = min(SR, n - strip * SR);
-      const int used = (ns + R - 1) / R;  // lanes holding read rows
-      const int lrows = lane < used ? min(R, ns - lane * R) : 0;
-      const int in0 = strip == 0 ? kLongStart : 0;  // exponent of the strip's input
-      if (g > 0 && strip < prof_len) {
-        // the first pair's decay of each lane, aiming its bottom at 2^0
-        const int d = lane < used ? (int)prof[strip * kWarp + lane] : 0;
-        klx = lane < used ? max(-96, min(120, d - (lane == 0 ? in0 : 0))) : 0;
-        kly = klx;
-      } else {
-        // the predicted boost spread evenly over the lanes holding read rows
-        klx = lane < used ? (lane + 1) * Bx / used - lane * Bx / used : 0;
-        kly = lane < used ? (lane + 1) * By / used - lane * By / used : 0;
-      }
-      for (int attempt = 0;; ++attempt) {
-        run_strip(strip, last);
-        if (qv.strip_runs != nullptr && lane == 0) {
-          atomicAdd(qv.strip_runs, 1ull);
-          if (attempt == 0) atomicAdd(qv.strip_runs + 1, 1ull);
-        }
-        const bool gx = !okx || (lgx >= kLongFloor && lgx < kLongCeil && lanes_in_window(lmx, used));
-        const bool gy = !oky || (lgy >= kLongFloor && lgy < kLongCeil && lanes_in_window(lmy, used));
-        if (gx && gy) break;
-        if (attempt + 1 == kLongTries) {
-          if (!gx) { okx = false; fail_x = true; }
-          if (!gy) { oky = false; fail_y = true; }
-          break;
-        }
-        // a half that left the window takes each lane's measured decay
-        if (!gx) klx = relane(klx, lmx, used, lrows, in0, lane);
-        if (!gy) kly = relane(kly, lmy, used, lrows, in0, lane);
-      }
-      // the strip's boost per half: the sum of its lanes' shares
-      Bx = klx;
-      By = kly;
+  // new exponents for the steps from t on, from the state, the lanes above and
+  // the staged inputs; `stage`: a window starts, its inputs go into the ring.
+  // INNER: no lane comes to a haplotype's end in these steps.
+  auto rescale = [&](auto inner_tag, const int t, const bool stage) {
+    constexpr bool INNER = decltype(inner_tag)::value;
+    if (last) {
+      add_total(accx, ex, totx, Ex);
+      add_total(accy, ey, toty, Ey);
+    }
+    // the lane below still holds this lane's last diagonal, in this lane's scale
+    float mx = __shfl_down_sync(FULL, s_top.x, 1), my = __shfl_down_sync(FULL, s_top.y, 1);
+    if (lane == kWarp - 1) mx = my = 0.f;
+    mx = fmaxf(mx, lane0 ? fmaxf(u_bot.x, s_top.x) : u_bot.x);
+    my = fmaxf(my, lane0 ? fmaxf(u_bot.y, s_top.y) : u_bot.y);
 #pragma unroll
-      for (int o = 16; o; o >>= 1) {
-        Bx += __shfl_xor_sync(FULL, Bx, o);
-        By += __shfl_xor_sync(FULL, By, o);
-      }
-      // a half whose read decayed by more than kLongMaxRate bits per row so far
-      // (with 64 bits of slack and the first strip's 2^60 start) is beyond what
-      // this tier keeps exact (alignment families that trade places across
-      // rows sit far below the row maximum): it goes to the drift and FP64 tiers
-      const int cap = kLongMaxRate * (Nrows + ns) + 64 + kLongStart;
-      if (okx && Dx + Bx + in0 - lgx > cap) { okx = false; fail_x = true; }
-      if (oky && Dy + By + in0 - lgy > cap) { oky = false; fail_y = true; }
-      if (g == 0 && strip == prof_len && strip < kLongProfStrips && (okx || oky)) {
-        const int lg = long_exponent(okx ? lmx : lmy);
-        int in = __shfl_up_sync(FULL, lg, 1);
-        if (lane == 0) in = in0;
-        prof[strip * kWarp + lane] = (short)(lane < used ? (okx ? klx : kly) + in - lg : 0);
-        ++prof_len;
-      }
-      // the boosts of the strip count into the exponent (plus the first strip's start)
-      if (!last) {
-        // the next strip reads this one's boundary brought to 2^0 (|lg| <= 60, so
-        // one exact factor); its boost is the read's mean decay rate so far
-        // times its rows
-        const int ksx = okx ? -lgx : 0, ksy = oky ? -lgy : 0;
-        inx = ksx;
-        iny = ksy;
-        const int ns1 = min(SR, n - (strip + 1) * SR);
-        Nrows += ns;
-        if (okx) {
-          Ex += Bx + in0 + ksx;
-          Dx += Bx + in0 - lgx;
-          Bx = max(0, min(4 * ns1, Dx * ns1 / Nrows));
-        }
-        if (oky) {
-          Ey += By + in0 + ksy;
-          Dy += By + in0 - lgy;
-          By = max(0, min(4 * ns1, Dy * ns1 / Nrows));
-        }
+    for (int r = 0; r < R; ++r) {
+      mx = fmaxf(mx, fmaxf(rw.s[r].x, rw.W[r].x));
+      my = fmaxf(my, fmaxf(rw.s[r].y, rw.W[r].y));
+    }
+    if (stage) {
+      // records past a haplotype's end do not count (nor do they lead anywhere)
+      const int p = t + lane;
+      in_x = __reduce_max_sync(FULL, INNER || p <= m1 ? state_exponent(fmaxf(nxt.x, nxt.y)) + nexp.x : kLongNone);
+      in_y = __reduce_max_sync(FULL, INNER || p <= m2 ? state_exponent(fmaxf(nxt.z, nxt.w)) + nexp.y : kLongNone);
+    }
+    const int ox = state_exponent(mx), oy = state_exponent(my);
+    // largest exponent the lane can reach in the coming steps.  A lane that
+    // has gone past the haplotype's last column feeds nothing any more.
+    auto bound = [&](int o, int e, int in, int mh) -> int {
+      int v = o + e;  // (far below every real one when there is nothing)
+      if (!INNER && t - 1 - lane > mh) v = kLongNone;
+      if (lane0 && (INNER || t <= mh)) v = max(v, in);
+      // far: the best of the lanes above less the bits lost on the way; h: the
+      // best of the lanes within reach by matches alone.  Near the haplotype's
+      // end fewer columns are left for matches: the other rows cost insertions.
+      // (A shuffle from above lane 0 returns the lane's own value.)
+      int far = v + cross, h = v;
+      if (!INNER) {
+        const int cols = min(SPAN, mh - (t - 1 - lane));
+        far -= row_bits * (SPAN - cols);
+#pragma unroll
+        for (int d = 1; d <= reach; ++d)
+          h = max(h, __shfl_up_sync(FULL, v - row_bits * max(0, R * (d - 1) + 1 - cols), d));
       } else {
-        Ex += Bx + in0;
-        Ey += By + in0;
+        int left = reach;
+#pragma unroll
+        for (int o2 = 1; o2 < kWarp; o2 <<= 1) {
+          if (left > 0) h = max(h, __shfl_up_sync(FULL, h, min(o2, left)));
+          left -= min(o2, left);
+        }
+      }
+#pragma unroll
+      for (int o2 = 1; o2 < kWarp; o2 <<= 1) far = max(far, __shfl_up_sync(FULL, far, o2));
+      far -= cross;
+      const int q = __shfl_up_sync(FULL, far, reach) + slack;
+      if (lane >= reach) h = max(h, q);
+      if (used < kWarp) {
+        // the lanes past the read pass u down the column unchanged
+        const int pad = __reduce_max_sync(FULL, lane >= used ? v : kLongNone);
+        const int end = __shfl_sync(FULL, h, used - 1);
+        if (lane >= used) h = max(pad, end);
+      }
+      return h;
+    };
+    const int Px = bound(ox, ex, in_x, m1), Py = bound(oy, ey, in_y, m2);
+    const int nx = Px > kLongNone / 2 ? Px - kLongTop : ex, ny = Py > kLongNone / 2 ? Py - kLongTop : ey;
+    int kx = ex - nx, ky = ey - ny;
+    float2 f;
+    // (nothing but denormals: they go to zero, whatever the new exponent)
+    const bool none_x = ox == kLongNone, none_y = oy == kLongNone;
+    const bool wide = __any_sync(FULL, (!none_x && abs(kx) > 126) || (!none_y && abs(ky) > 126));
+    f = make_float2(none_x ? 0.f : pow2T(kx, 0.f), none_y ? 0.f : pow2T(ky, 0.f));
+    if (wide) {
+      // a shift beyond one factor: halve it (what needs more than 2^252 is zero)
+      kx = none_x ? -252 : max(-252, min(252, kx));
+      ky = none_y ? -252 : max(-252, min(252, ky));
+      f = make_float2(pow2T(kx / 2, 0.f), pow2T(ky / 2, 0.f));
+      const float2 f2 = make_float2(pow2T(kx - kx / 2, 0.f), pow2T(ky - ky / 2, 0.f));
+      float2 g2 = make_float2(__shfl_up_sync(FULL, f2.x, 1), __shfl_up_sync(FULL, f2.y, 1));
+      s_top = __fmul2_rn(s_top, g2);  // (lane 0: its own)
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        rw.W[r] = __fmul2_rn(rw.W[r], f2);
+        rw.s[r] = __fmul2_rn(rw.s[r], f2);
+      }
+      u_bot = __fmul2_rn(u_bot, f2);
+    }
+    // s_top came from the lane above (lane 0: from the ring, in its own scale)
+    s_top = __fmul2_rn(s_top, make_float2(__shfl_up_sync(FULL, f.x, 1), __shfl_up_sync(FULL, f.y, 1)));
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      rw.W[r] = __fmul2_rn(rw.W[r], f);
+      rw.s[r] = __fmul2_rn(rw.s[r], f);
+    }
+    u_bot = __fmul2_rn(u_bot, f);
+    // the window's inputs in lane 0's scale
+    const int e0x = __shfl_sync(FULL, nx, 0), e0y = __shfl_sync(FULL, ny, 0);
+    __syncwarp();
+    if (stage) {
+      const int sx = nexp.x - e0x, sy = nexp.y - e0y;
+      ring[lane] = make_float4(scale2(nxt.x, sx), scale2(nxt.y, sx), scale2(nxt.z, sy), scale2(nxt.w, sy));
+    } else {
+      const int sx = __shfl_sync(FULL, ex, 0) - e0x, sy = __shfl_sync(FULL, ey, 0) - e0y;
+      if (sx != 0 || sy != 0) {
+        const float4 raw = ring[lane];
+        ring[lane] = make_float4(scale2(raw.x, sx), scale2(raw.y, sx), scale2(raw.z, sy), scale2(raw.w, sy));
       }
     }
-
-    // ln of the final sum z = f 2^e (f in [1/2, 1)) less the boosts: the bits
-    // do not depend on which powers of two the boosts took
+    ex = nx;
+    ey = ny;
+    // inputs come in the scale of the lane above: fold the difference into row 0
+    const int upx = __shfl_up_sync(FULL, ex, 1) - ex, upy = __shfl_up_sync(FULL, ey, 1) - ey;  // (lane 0: 0)
+    const float2 in = make_float2(pow2T(max(-127, min(126, upx)), 0.f), pow2T(max(-127, min(126, upy)), 0.f));
+    rw.hit0 = in;
+    rw.miss0 = make_float2(rw.miss[0] * in.x, rw.miss[0] * in.y);
+    rw.K[0] = make_float2(K0 * in.x, K0 * in.y);
+    rw.X[0] = make_float2(X0 * in.x, X0 * in.y);
     if (lane == kWarp - 1) {
-      const int64_t o1 = w.out_begin + g;
-      if (okx && !fail_x) {
-        int e;
-        const double f = frexp(zx, &e);
-        bv.out[o1] = log(f) - (sc.ln_c + log((double)(m1 + 1))) + lnN + (double)(e - Ex) * kLn2;
-      } else {
-        bv.out[o1] = __longlong_as_double(0x7ff8000000000000LL);
-        spill_pair<float>(qv, w.read, h1, o1);
-      }
-      if (two) {
-        if (oky && !fail_y) {
-          int e;
-          const double f = frexp(zy, &e);
-          bv.out[o1 + 1] = log(f) - (sc.ln_c + log((double)(m2 + 1))) + lnN + (double)(e - Ey) * kLn2;
-        } else {
-          bv.out[o1 + 1] = __longlong_as_double(0x7ff8000000000000LL);
-          spill_pair<float>(qv, w.read, h2, o1 + 1);
-        }
-      }
+      const int q = (t >> 3) & 3;
+      oexp[q] = make_int2(ex, ey);
+      if (SPAN == 16) oexp[q + 1] = make_int2(ex, ey);
     }
     __syncwarp();
+  };
+
+  const float2 k2 = make_float2(sc.k2, sc.k2), x = make_float2(sc.x, sc.x);
+  // one step; STEADY: every lane at a column in 1 .. min(m1, m2), its bases given
+  auto step = [&](auto steady_tag, const int t, uint32_t hbx, uint32_t hby) {
+    constexpr bool STEADY = decltype(steady_tag)::value;
+    const int p = t - lane;  // this lane's column
+    const float4 rec = ring[t & (kWarp - 1)];
+    if (!STEADY) {
+      // before column 1 the base does not matter (the state and the diagonal
+      // are zero); past a haplotype's end its columns are not used
+      hbx = __ldg(hp1 + max(1, min(p, m1)));
+      hby = __ldg(hp2 + max(1, min(p, m2)));
+    }
+    float2 u_in = shfl_up2(u_bot);
+    float2 s_in = shfl_up2(rw.s[R - 1]);
+    u_in = lane0 ? make_float2(rec.y, rec.w) : u_in;
+    s_in = lane0 ? make_float2(rec.x, rec.z) : s_in;
+    column_long<R>(rw, hbx, hby, s_top, u_in, k2, x, u_bot);
+    s_top = s_in;
+    if (STEADY) {
+      acc32 = __fadd2_rn(acc32, u_bot);
+    } else if (p >= 0) {
+      if (p <= m1) acc32.x += u_bot.x;
+      if (p <= m2) acc32.y += u_bot.y;
+    }
+    if (lane == kWarp - 1) oring[t & (kWarp - 1)] = make_float4(rw.s[R - 1].x, u_bot.x, rw.s[R - 1].y, u_bot.y);
+  };
+  // the FP32 row sums move into FP64 every 8 steps
+  auto flush_acc = [&]() {
+    if (last) {
+      accx += (double)acc32.x;
+      accy += (double)acc32.y;
+    }
+    acc32 = make_float2(0.f, 0.f);
+  };
+  // the 8 bases a lane passes in a group, as three aligned words (their first
+  // and last bytes may belong to a neighbour in the batch's haplotype buffer),
+  // loaded a group ahead
+  uint32_t px0 = 0, px1 = 0, px2 = 0, py0 = 0, py1 = 0, py2 = 0;
+  int fetched = -1;
+  auto fetch = [&](const int t) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(hp1 + (t - lane)), b = reinterpret_cast<uintptr_t>(hp2 + (t - lane));
+    const uint32_t* qa = reinterpret_cast<const uint32_t*>(a & ~(uintptr_t)3);
+    const uint32_t* qb = reinterpret_cast<const uint32_t*>(b & ~(uintptr_t)3);
+    px0 = __ldg(qa);
+    px1 = __ldg(qa + 1);
+    px2 = __ldg(qa + 2);
+    py0 = __ldg(qb);
+    py1 = __ldg(qb + 1);
+    py2 = __ldg(qb + 2);
+    fetched = t;
+  };
+  auto group = [&](auto steady_tag, const int wn, const int q) {
+    const int t = wn * kWarp + q * 8;
+    if constexpr (decltype(steady_tag)::value) {
+      if (fetched != t) fetch(t);
+      if (((q * 8) & (SPAN - 1)) == 0) rescale(steady_tag, t, q == 0);
+      const int sx = ((int)reinterpret_cast<uintptr_t>(hp1) + t - lane) & 3, sy = ((int)reinterpret_cast<uintptr_t>(hp2) + t - lane) & 3;
+      const uint32_t xa = __funnelshift_r(px0, px1, sx * 8), xb = __funnelshift_r(px1, px2, sx * 8);
+      const uint32_t ya = __funnelshift_r(py0, py1, sy * 8), yb = __funnelshift_r(py1, py2, sy * 8);
+      // (the next group's columns lie inside both haplotypes, or are not used)
+      if (t + 15 <= min(m1, m2)) fetch(t + 8);
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        step(steady_tag, t + u, __byte_perm(u < 4 ? xa : xb, 0, 0x4440 + (u & 3)),
+             __byte_perm(u < 4 ? ya : yb, 0, 0x4440 + (u & 3)));
+    } else {
+      if (((q * 8) & (SPAN - 1)) == 0) rescale(steady_tag, t, q == 0);
+#pragma unroll 1
+      for (int u = 0; u < 8; ++u) step(steady_tag, t + u, 0u, 0u);
+    }
+    flush_acc();
+    // the block laid down at the end of the last window: its stores have long
+    // arrived, so the release costs no wait
+    if (q == 0 && !last && lane0 && wn > 0) st_release(word, tag | (unsigned)wn);
+    if (q == 1 && !first && wn + 1 < nwin) load_window(wn + 1);
+  };
+  for (int wn = 0; wn < nwin; ++wn) {
+    // columns of this window: 32 wn - 31 .. 32 wn + 31
+    if (wn >= 1 && wn * kWarp + kWarp - 1 <= min(m1, m2)) {
+#pragma unroll 1
+      for (int q = 0; q < kWarp / 8; ++q) group(std::true_type{}, wn, q);
+    } else {
+#pragma unroll 1
+      for (int q = 0; q < kWarp / 8; ++q) group(std::false_type{}, wn, q);
+    }
+    if (!ok) return false;
+    if (!last) {
+      // block wn: columns 32 (wn - 1) + 1 .. 32 wn, 8 columns to an exponent
+      __syncwarp();
+      const int p = (wn - 1) * kWarp + 1 + lane;
+      const int2 e = oexp[lane >> 3];
+      if (p >= 0 && p <= M) {
+        const float4 rec = oring[lane];
+        __stcg(dst + p, rec);
+        if (p <= m1) bmx = max(bmx, state_exponent(fmaxf(rec.x, rec.y)) + e.x);
+        if (p <= m2) bmy = max(bmy, state_exponent(fmaxf(rec.z, rec.w)) + e.y);
+      }
+      if ((lane & 7) == 0) __stcg(dst_exp + wn * (kWarp / 8) + (lane >> 3), e);
+      __syncwarp();
+    }
   }
+  if (last) {
+    add_total(accx, ex, totx, Ex);
+    add_total(accy, ey, toty, Ey);
+  }
+
+  // the halves that left what this tier keeps: their decay so far is over the rate
+  unsigned failed = 0;
+  if (!first) {
+    const unsigned long long v = wait_task(above, nwin, err, ok);
+    if (!ok) return false;
+    failed = task_fail(v);
+  }
+  const int cap = long_max_bits(min(n, i0 + SR));
+  if (!last) {
+    bmx = __reduce_max_sync(FULL, bmx);
+    bmy = __reduce_max_sync(FULL, bmy);
+    if (bmx < -cap) failed |= 1u;
+    if (bmy < -cap) failed |= 2u;
+    __syncwarp();
+    if (lane0) {
+      __threadfence();
+      st_release(word, tag | ((unsigned long long)failed << 30) | (unsigned)nwin);
+    }
+  } else {
+    double lnN = 0.0;
+    for (int i = lane; i < n; i += kWarp) lnN += tb->lnN[rqual[i]];
+#pragma unroll
+    for (int o = 16; o; o >>= 1) lnN += __shfl_xor_sync(FULL, lnN, o);
+    if (lane == kWarp - 1) {
+      // ln of the final sum z = f 2^e (f in [1/2, 1)) and the exponent
+      auto write = [&](double z, int E, bool bad, int m, int64_t h, int64_t o) {
+        int e = 0;
+        const double f = frexp(z, &e);
+        if (!bad && z > 0.0 && z < HUGE_VAL && e - 1 + E >= -cap) {
+          bv.out[o] = log(f) - (sc.ln_c + log((double)(m + 1))) + lnN + (double)(e + E) * kLn2;
+        } else {
+          bv.out[o] = __longlong_as_double(0x7ff8000000000000LL);
+          spill_pair<float>(qv, w.read, h, o);
+        }
+      };
+      write(totx, Ex, (failed & 1u) != 0, m1, h1, w.out_begin + g);
+      if (two) write(toty, Ey, (failed & 2u) != 0, m2, h2, w.out_begin + g + 1);
+    }
+    if (lane0) st_release(word, (unsigned)nwin);
+  }
+  if (qv.strip_runs != nullptr && lane0) {
+    atomicAdd(qv.strip_runs, 1ull);
+    atomicAdd(qv.strip_runs + 1, 1ull);
+  }
+  return true;
 }
 
-// Persistent kernel of the long-read items (FP32 semiglobal primary tier):
-// every warp pulls items from qv.head (or walks them in the fixed round-robin
-// order of the plain schedule).  Items whose read has another rows-per-lane
-// count than R are not in its list.
-template <int R, int kBlocks>
+// Persistent kernel of the long-read items (FP32 semiglobal primary tier): the
+// warps pull tasks (strips of pairs) in order from qv.head, in both schedules.
+// qv.long_off[i] is the number of item i's first task.  Each warp owns two
+// boundary buffers and alternates; a buffer is written again once the task
+// that reads it is done.
+template <int LO, int HI, int kBlocks, int SPAN>
 __global__ void __launch_bounds__(kWarpsPerBlock * kWarp, kBlocks)
-pairhmm_long_kernel(const BatchView bv, const QueueView qv, const Tables<float>* __restrict__ gtab,
-                    const Scalars<float> sc) {
+pairhmm_long_kernel(const __grid_constant__ BatchView bv, const __grid_constant__ QueueView qv,
+                    const Tables<float>* __restrict__ gtab, const __grid_constant__ Scalars<float> sc) {
+  constexpr unsigned FULL = 0xffffffffu;
   __shared__ Tables<float> tab;
   __shared__ float4 rings[kWarpsPerBlock][2][kWarp];
-  __shared__ short profs[kWarpsPerBlock][kLongProfStrips * kWarp];
+  __shared__ int2 exps[kWarpsPerBlock][4];
   {
     const int words = (int)(sizeof(Tables<float>) / sizeof(int));
     const int* src = reinterpret_cast<const int*>(gtab);
@@ -546,23 +653,56 @@ pairhmm_long_kernel(const BatchView bv, const QueueView qv, const Tables<float>*
     for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
   }
   __syncthreads();
-  const int lane = threadIdx.x & (kWarp - 1);
-  const long long gw = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-  float4* scratch = reinterpret_cast<float4*>(qv.scratch) + gw * qv.scratch_stride;
-  const long long stride = (long long)gridDim.x * kWarpsPerBlock;
-  long long next = gw;
-  for (;;) {
-    unsigned long long i = 0;
-    if (qv.static_order) {
-      i = (unsigned long long)next;
-      next += stride;
-    } else {
-      if (lane == 0) i = atomicAdd(qv.head, 1ull);
-      i = __shfl_sync(0xffffffffu, i, 0);
+  const int lane = threadIdx.x & (kWarp - 1), wid = threadIdx.x >> 5;
+  const int gw = (int)(blockIdx.x * kWarpsPerBlock) + wid;
+  float4* const bufs = reinterpret_cast<float4*>(qv.scratch);
+  const long long half = qv.scratch_stride / 2;
+  long long reader[2] = {-1, -1};  // per buffer: the task that reads what this warp last wrote there
+  int reader_blocks[2] = {0, 0};   // and its blocks
+  for (int turn = 0;; turn ^= 1) {
+    unsigned long long k = 0;
+    if (lane == 0) k = atomicAdd(qv.head, 1ull);
+    k = __shfl_sync(FULL, k, 0);
+    if ((long long)k >= qv.long_tasks) break;
+    // the item: the last one whose first task is not past k (32-way search)
+    long long lo = 0, hi = qv.n_items;
+    while (hi - lo > 1) {
+      const long long st = (hi - lo + kWarp - 1) / kWarp;
+      const long long at = lo + lane * st;
+      const unsigned b = __ballot_sync(FULL, at < hi && qv.long_off[at] <= (long long)k);
+      const int c = __popc(b) - 1;
+      lo += c * st;
+      hi = min(hi, lo + st);
     }
-    if ((long long)i >= qv.n_items) break;
-    process_long<R>(bv, qv, qv.items[i], &tab, sc, lane, scratch, rings[threadIdx.x >> 5][0],
-                    rings[threadIdx.x >> 5][1], profs[threadIdx.x >> 5]);
+    const WorkItem w = qv.items[lo];
+    const int R = code_R(w.code);
+    const int n = (int)(bv.read_off[w.read + 1] - bv.read_off[w.read]);
+    const int nstrips = (n + kWarp * R - 1) / (kWarp * R);
+    const int j = (int)((long long)k - qv.long_off[lo]);
+    const int g = 2 * (j / nstrips), strip = j % nstrips;
+    bool ok = true;
+    if (strip < nstrips - 1) {
+      if (reader[turn] >= 0) wait_task(qv.long_words + reader[turn], reader_blocks[turn], qv.error_flag, ok);
+      const int64_t h = w.hap_begin + g;
+      const int ma = (int)(bv.hap_off[h + 1] - bv.hap_off[h]);
+      const int mb = g + 1 < w.nhap ? (int)(bv.hap_off[h + 2] - bv.hap_off[h + 1]) : ma;
+      reader[turn] = (long long)k + 1;
+      reader_blocks[turn] = (max(ma, mb) + kWarp - 1) / kWarp + 1;
+    }
+    if (ok) {
+      switch (R) {
+#define VD_LCASE(r)                                                                                              \
+  case r:                                                                                                        \
+    if constexpr (r >= LO && r <= HI)                                                                            \
+      ok = long_task<r, SPAN>(bv, qv, w, g, strip, nstrips, (long long)k, &tab, sc, lane, bufs, half, 2 * gw + turn,  \
+                        rings[wid][0], rings[wid][1], exps[wid]);                                                        \
+    break;
+        VD_LCASE(4) VD_LCASE(5) VD_LCASE(6) VD_LCASE(7) VD_LCASE(8)
+#undef VD_LCASE
+        default: break;
+      }
+    }
+    if (!__all_sync(FULL, ok)) break;  // a wait gave up: the error flag is set
   }
 }
 

@@ -13,8 +13,14 @@ cudaError_t launch_long_f32(int R, bool block, const BatchView& bv, const QueueV
     if (R == 8) pairhmm_long_block_kernel<8, 3><<<grid, threads, 0, stream>>>(bv, qv, tab, sc);
     else pairhmm_long_block_kernel<4, 4><<<grid, threads, 0, stream>>>(bv, qv, tab, sc);
   } else {
-    if (R == 8) pairhmm_long_kernel<8, 3><<<grid, threads, 0, stream>>>(bv, qv, tab, sc);
-    else pairhmm_long_kernel<4, 4><<<grid, threads, 0, stream>>>(bv, qv, tab, sc);
+    // (gap continuations below 0.08 choose the lanes' exponents twice as often)
+    if (sc.x >= 0.08f) {
+      if (R == 8) pairhmm_long_kernel<5, 8, 3, kLongSpan><<<grid, threads, 0, stream>>>(bv, qv, tab, sc);
+      else pairhmm_long_kernel<4, 4, 4, kLongSpan><<<grid, threads, 0, stream>>>(bv, qv, tab, sc);
+    } else {
+      if (R == 8) pairhmm_long_kernel<5, 8, 3, kLongSpanShort><<<grid, threads, 0, stream>>>(bv, qv, tab, sc);
+      else pairhmm_long_kernel<4, 4, 4, kLongSpanShort><<<grid, threads, 0, stream>>>(bv, qv, tab, sc);
+    }
   }
   return cudaGetLastError();
 }
@@ -24,8 +30,8 @@ cudaError_t occupancy_long_f32(int R, bool block, int* blocks_per_sm) {
   if (block)
     return R == 8 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, pairhmm_long_block_kernel<8, 3>, threads, 0)
                   : cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, pairhmm_long_block_kernel<4, 4>, threads, 0);
-  return R == 8 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, pairhmm_long_kernel<8, 3>, threads, 0)
-                : cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, pairhmm_long_kernel<4, 4>, threads, 0);
+  return R == 8 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, pairhmm_long_kernel<5, 8, 3, kLongSpan>, threads, 0)
+                : cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, pairhmm_long_kernel<4, 4, 4, kLongSpan>, threads, 0);
 }
 
 }  // namespace vd
