@@ -311,6 +311,7 @@ struct BuildOpts {
   int pair_split = 6;              // two-read items with this many rows per lane or more: 12-warp kernel
   int pair_mask = 0x1fe;           // bit R: two reads of R rows per lane may share a warp
   int64_t max_stream = 1 << 30;    // haplotype columns one work item streams at most
+  int64_t item_limit = INT64_MAX;  // work (item_work) from which an item is cut between haplotypes
 };
 
 // Rows per lane for a read of n rows: the smallest R with 32 R >= n, at most
@@ -340,6 +341,51 @@ BuildOpts build_opts(const vd_engine* e) {
   bo.long_group = bo.long_block ? 2 : e->tuning.long_group > 0 ? e->tuning.long_group : kLongGroupMax;
   bo.pair_split = e->tuning.pair_split == 7 ? 7 : 6;
   return bo;
+}
+
+
+// Work of an item in lane-row steps: every column step of the stream costs its
+// R rows and about two more for the shuffles and the bookkeeping.
+inline int64_t item_work(int64_t stream, int R) { return (stream + kWarp) * (R + 2); }
+
+// The most work one item of a batch may hold: a quarter of what each of the
+// resident warps (12 per SM) gets of the batch's one-strip reads, two reads to
+// a warp where they are packed.  The persistent warps then finish within a
+// quarter of their load of each other however small the batch, and a batch that
+// gives every warp many items is not cut at all.  60 regions (6.7e9 cells; the
+// largest item was 16 haplotypes of 1,000 columns): kernels 6.5 -> 2.5 ms; 40 in
+// FP64 2.3 -> 1.4, one of 64 reads 0.136 -> 0.104.  Shares of 1/2, 1/4, 1/8 and 1/16
+// ran the 60 regions in 3.7, 2.5, 2.3 and 2.2 ms, but every item costs the host
+// some 45 ns, and the whole call took 7.9, 6.9, 7.1 and 7.3 ms.  It is taken over the whole
+// batch, so that the items, and the prefixes they share, do not depend on the
+// pipeline's chunks.
+int64_t batch_item_limit(const vd_engine* e, const vd_batch* b, const vd_params* p) {
+  auto rows = [&](int64_t r) -> int64_t {
+    const int64_t n = b->read_off[r + 1] - b->read_off[r];
+    return n <= 0 || n + p->anchored > kStripRows ? 0 : rows_per_lane((int)n + p->anchored) + 2;
+  };
+  std::atomic<int64_t> sum{0};
+  if (b->pair_read) {
+    parallel_for(b->n_pairs, 65536, [&](int64_t lo, int64_t hi) {
+      int64_t s = 0;
+      for (int64_t q = lo; q < hi; ++q) s += rows(b->pair_read[q]) * (b->hap_off[b->pair_hap[q] + 1] - b->hap_off[b->pair_hap[q]]);
+      sum += s;
+    });
+  } else {
+    parallel_for(b->n_regions, 256, [&](int64_t lo, int64_t hi) {
+      int64_t s = 0;
+      for (int64_t g = lo; g < hi; ++g) {
+        int64_t k = 0;
+        for (int64_t r = b->region_read_off[g]; r < b->region_read_off[g + 1]; ++r) k += rows(r);
+        s += k * (b->hap_off[b->region_hap_off[g + 1]] - b->hap_off[b->region_hap_off[g]] + kWarp);
+      }
+      sum += s;
+    });
+  }
+  const bool packed = !b->pair_read && !p->anchored && p->precision == VD_PRECISION_MIXED;
+  // (items of 256 columns at 8 rows, or as much work, are never cut: below that
+  // the ramp and the host's share outweigh the balance)
+  return std::max<int64_t>(item_work(256, kMaxR), sum.load() / (packed ? 8 : 4) / std::max<int64_t>(1, (int64_t)e->sm_count * 12));
 }
 
 
@@ -668,6 +714,8 @@ void build_region_chunk(const vd_batch* b, int64_t g0, int64_t g1, const TableSe
           // columns past its shared prefix
           const int col0 = (sorted && run_end > h) ? c.hap_share[run_end - c.ha] + 1 : 0;
           if (run_end > h && (plain || multistrip || stream + m + 1 - col0 > kMaxStream)) break;
+          // over the limit: cut, unless the haplotype shares most of its columns
+          if (run_end > h && item_work(stream + m + 1 - col0, R) > bo.item_limit && 2 * col0 <= m) break;
           stream += m + 1 - col0;
           sl.cells += (int64_t)(n + n2) * m;
           if (col0 > 0) sl.shared += (int64_t)(n + n2) * (col0 - 1);
@@ -817,7 +865,7 @@ void build_pair_chunk(const vd_batch* b, const PairGroups& pg, int64_t ra, int64
         // stays -inf: out_sel keeps no entry for it
         continue;
       }
-      if (stream > 0 && (multistrip || stream + m + 1 > kMaxStream)) flush();
+      if (stream > 0 && (multistrip || stream + m + 1 > kMaxStream || item_work(stream + m + 1, R) > bo.item_limit)) flush();
       c.hap_sel.push_back((int32_t)h);
       c.out_sel.push_back(slot);
       stream += m + 1;
@@ -1489,7 +1537,8 @@ int vd_forward(vd_engine* e, const vd_batch* b, const vd_params* p, double* out,
   for (int64_t u = 0; u < units; ++u) total_cells += unit_cells(u);
   // warp items of the long-read kernel (reads longer than a strip, up to
   // long_group haplotypes each)
-  const BuildOpts lbo = build_opts(e);
+  BuildOpts lbo = build_opts(e);
+  lbo.item_limit = batch_item_limit(e, b, p);
   int64_t long_items = 0;
   if (lbo.long_warp && !lbo.long_block && p->precision != VD_PRECISION_FLOAT64 && !p->anchored) {
     auto long_reads = [&](int64_t r0, int64_t r1) {
@@ -1582,7 +1631,7 @@ int vd_forward(vd_engine* e, const vd_batch* b, const vd_params* p, double* out,
     pl.ev_join = sl.join;
     const double th = now_ms();
     const bool plain = p->schedule == VD_SCHEDULE_PLAIN;
-    const BuildOpts bo = build_opts(e);
+    const BuildOpts& bo = lbo;
     if (pair_form) build_pair_chunk(b, pg, u, u_end, e->htab, offsets, p->anchored != 0, pl.chunk, plain, bo);
     else build_region_chunk(b, u, u_end, e->htab, offsets, p->anchored != 0, p->precision == VD_PRECISION_MIXED,
                             pl.chunk, plain, bo);
@@ -1651,7 +1700,8 @@ int vd_plan_create(vd_engine* e, const vd_batch* b, const vd_params* p, vd_plan*
   }
   const bool offsets = p->quality_offsets != nullptr;
   const bool plain = p->schedule == VD_SCHEDULE_PLAIN;
-  const BuildOpts bo = build_opts(e);
+  BuildOpts bo = build_opts(e);
+  bo.item_limit = batch_item_limit(e, b, p);
   if (b->pair_read) {
     PairGroups pg;
     group_pairs(b, pg);

@@ -142,12 +142,16 @@ __global__ void na_prep_reads(const unsigned char* __restrict__ read_quals, cons
   }
 }
 
-// Primary tier over the region: work item r is read r against the non-empty
-// haplotypes, derived here instead of read from a host-built list.
+// Primary tier over the region: work item i is read i / pieces against its share
+// of the non-empty haplotypes (the (i mod pieces)-th of `pieces` runs), derived
+// here instead of read from a host-built list.  Reads alone leave most of the
+// GPU idle (301 reads x 13 haplotypes of 421 bases: 1.10 ms with one item per
+// read, a serial chain of 5,500 columns); the call asks for about four items
+// per resident warp.
 template <typename T, bool ANCH>
 __global__ void __launch_bounds__(kWarpsPerBlock * kWarp, MinBlocks<T>::value)
 na_primary(const __grid_constant__ BatchView bv, const __grid_constant__ QueueView qv,
-           const __grid_constant__ Scalars<T> sc, int n_reads, unsigned char* scratch) {
+           const __grid_constant__ Scalars<T> sc, int n_reads, int pieces, unsigned char* scratch) {
   __shared__ Tables<T> tab;
   {
     const Tables<T>* g = reinterpret_cast<const Tables<T>*>(scratch + (sizeof(T) == 4 ? kOffTab32 : kOffTab64));
@@ -167,15 +171,17 @@ na_primary(const __grid_constant__ BatchView bv, const __grid_constant__ QueueVi
     unsigned long long i = 0;
     if (lane == 0) i = atomicAdd(qv.head, 1ull);
     i = __shfl_sync(0xffffffffu, i, 0);
-    if ((long long)i >= n_reads) break;
-    const int n = (int)(bv.read_off[i + 1] - bv.read_off[i]);
-    if (n <= 0 || nh_ne == 0) continue;
+    if ((long long)i >= (long long)n_reads * pieces) break;
+    const int r = (int)(i / pieces), piece = (int)(i % pieces);
+    const int n = (int)(bv.read_off[r + 1] - bv.read_off[r]);
+    const int h0 = (int)((long long)nh_ne * piece / pieces), h1 = (int)((long long)nh_ne * (piece + 1) / pieces);
+    if (n <= 0 || h1 <= h0) continue;
     ItemRef it;
-    it.w.read = (int32_t)i;
-    it.w.nhap = nh_ne;
-    it.w.hap_begin = 0;
-    it.w.out_begin = (int64_t)i * nh_ne;
-    it.w.code = bv.read_code[i];
+    it.w.read = r;
+    it.w.nhap = h1 - h0;
+    it.w.hap_begin = h0;
+    it.w.out_begin = (int64_t)r * nh_ne + h0;
+    it.w.code = bv.read_code[r];
     it.w.read2 = -1;
     it.w.out2_begin = 0;
     it.use_sel = true;
@@ -357,12 +363,14 @@ extern "C" int vd_forward_region_noalloc(int device, const unsigned char* read_b
   q.scratch_stride = kNaMaxHapLen + 1;
   q.error_flag = reinterpret_cast<int*>(cnt + 5);
   // primary tier: FP32 (or FP64 when asked), work items derived on the device
+  const int64_t warps = (int64_t)(f64 ? d.grid64 : d.grid32)[anch] * kWarpsPerBlock;
+  const int pieces = (int)std::max<int64_t>(1, std::min<int64_t>(n_haps, 4 * warps / n_reads));
   if (f64) {
-    if (anch) na_primary<double, true><<<d.grid64[1], kWarpsPerBlock * kWarp, 0, s>>>(bv, q, s64, (int)n_reads, sc);
-    else na_primary<double, false><<<d.grid64[0], kWarpsPerBlock * kWarp, 0, s>>>(bv, q, s64, (int)n_reads, sc);
+    if (anch) na_primary<double, true><<<d.grid64[1], kWarpsPerBlock * kWarp, 0, s>>>(bv, q, s64, (int)n_reads, pieces, sc);
+    else na_primary<double, false><<<d.grid64[0], kWarpsPerBlock * kWarp, 0, s>>>(bv, q, s64, (int)n_reads, pieces, sc);
   } else {
-    if (anch) na_primary<float, true><<<d.grid32[1], kWarpsPerBlock * kWarp, 0, s>>>(bv, q, s32, (int)n_reads, sc);
-    else na_primary<float, false><<<d.grid32[0], kWarpsPerBlock * kWarp, 0, s>>>(bv, q, s32, (int)n_reads, sc);
+    if (anch) na_primary<float, true><<<d.grid32[1], kWarpsPerBlock * kWarp, 0, s>>>(bv, q, s32, (int)n_reads, pieces, sc);
+    else na_primary<float, false><<<d.grid32[0], kWarpsPerBlock * kWarp, 0, s>>>(bv, q, s32, (int)n_reads, pieces, sc);
   }
   NA_CUDA(cudaGetLastError());
   // rescue tiers on the spill lists, with the library's own kernels
