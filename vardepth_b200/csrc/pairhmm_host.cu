@@ -170,6 +170,35 @@ struct DevBuf {
 
 }  // namespace
 
+// Streams beside a plan's or a slot's own, forked from it and joined into it: the
+// primary tier's kernels run on them side by side.  Each is persistent and fills
+// the SMs by itself, so kernels of a lower stream priority start as the blocks of
+// the higher ones run out of items: they fill each other's tails (priorities
+// order the blocks waiting to start; s[0] is above the plan's own stream, s[1]
+// below).
+constexpr int kOwnPriority = -1;
+struct SideStreams {
+  cudaStream_t s[2] = {nullptr, nullptr};
+  cudaEvent_t fork = nullptr, join[2] = {nullptr, nullptr};
+  cudaError_t create() {
+    cudaError_t err = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
+    for (int k = 0; k < 2 && err == cudaSuccess; ++k)
+      if ((err = cudaStreamCreateWithPriority(&s[k], cudaStreamNonBlocking, kOwnPriority + (k ? 1 : -1))) ==
+          cudaSuccess)
+        err = cudaEventCreateWithFlags(&join[k], cudaEventDisableTiming);
+    return err;
+  }
+  void synchronize() {
+    for (cudaStream_t x : s) if (x) cudaStreamSynchronize(x);
+  }
+  void destroy() {
+    if (fork) cudaEventDestroy(fork);
+    for (cudaEvent_t& x : join) if (x) cudaEventDestroy(x);
+    for (cudaStream_t& x : s) if (x) cudaStreamDestroy(x);
+    *this = SideStreams();
+  }
+};
+
 // ---- engine -----------------------------------------------------------------------
 
 struct vd_engine {
@@ -180,10 +209,7 @@ struct vd_engine {
   size_t budget = 0;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev_begin = nullptr, ev_mid = nullptr, ev_end = nullptr;
-  // the long-read kernel runs on a side stream beside the other primary
-  // kernels: as its persistent blocks run out of items, theirs take the SMs
-  cudaStream_t side = nullptr;
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+  SideStreams side;
   std::mutex mu;
   int grid[2][2] = {{0, 0}, {0, 0}};  // [f64][anchored] blocks
   int grid_pair[2][2] = {{0, 0}, {0, 0}};  // blocks of the two-read kernels [split == 7][wide]
@@ -207,9 +233,9 @@ struct vd_engine {
   // so one chunk's host work-list build and upload overlap the other's kernels
   struct Slot {
     DevBuf arena;
-    cudaStream_t stream = nullptr, side = nullptr;
+    cudaStream_t stream = nullptr;
+    SideStreams side;
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
-    cudaEvent_t fork = nullptr, join = nullptr;
     unsigned long long* hcnt = nullptr;  // pinned copy of the tier counters
     std::vector<double> stage;           // pair-form outputs before the scatter
     vd_plan* pl = nullptr;
@@ -989,8 +1015,7 @@ struct vd_plan {
   // or a pipeline slot's in vd_forward)
   cudaStream_t stream = nullptr;
   cudaEvent_t ev_begin = nullptr, ev_mid = nullptr, ev_end = nullptr;
-  cudaStream_t side = nullptr;                        // the long-read kernel's stream
-  cudaEvent_t ev_fork = nullptr, ev_join = nullptr;  // its fork from and join into `stream`
+  SideStreams* side = nullptr;                        // the streams beside it
   int64_t last_rescued1 = 0, last_rescued2 = 0;
 };
 
@@ -1092,12 +1117,17 @@ int enqueue_tiers(vd_plan* pl, int* launches, bool capturing = false) {
     const int64_t np = pl->chunk.n_paired, nw = pl->chunk.n_paired_wide;
     const int64_t nl = pl->chunk.n_long;
     q.static_order = pl->params.schedule == VD_SCHEDULE_PLAIN ? 1 : 0;
+    const int64_t ns = (int64_t)pl->chunk.items.size() - np - nl;
+    // up to four kernels, each persistent: the long reads on one side stream, the
+    // narrow two-read items on the other (with the plan's own stream free they
+    // take that), the wide two-read items and then the single reads on the plan's
+    const bool narrow_aside = np > nw && (nw > 0 || ns > 0);
+    if (nl > 0 || narrow_aside) VD_CUDA(cudaEventRecord(pl->side->fork, pl->stream));
     if (nl > 0) {
-      // long reads, a warp per strip of a pair of haplotypes, launched first on
-      // the side stream: the kernels below take the SMs its blocks leave as its
-      // queue runs dry, so they fill its tail; its failures join the spill list
-      VD_CUDA(cudaEventRecord(pl->ev_fork, pl->stream));
-      VD_CUDA(cudaStreamWaitEvent(pl->side, pl->ev_fork, 0));
+      // long reads, a warp per strip of a pair of haplotypes, launched first: the
+      // kernels below take the SMs its blocks leave as its queue runs dry; its
+      // failures join the spill list
+      VD_CUDA(cudaStreamWaitEvent(pl->side->s[0], pl->side->fork, 0));
       QueueView ql = q;
       ql.items = (const WorkItem*)(d + L.o_items) + np;
       ql.n_items = nl;
@@ -1111,13 +1141,13 @@ int enqueue_tiers(vd_plan* pl, int* launches, bool capturing = false) {
       ql.long_exp_off = pl->chunk.max_hap + 1;
       const int R = pl->chunk.long_R;
       const bool blk = pl->chunk.long_block;
-      err = launch_long_f32(R, blk, bv, ql, &dt->f32, ht->s32d, e->grid_long[blk ? 1 : 0][R == 8 ? 1 : 0], pl->side);
+      err = launch_long_f32(R, blk, bv, ql, &dt->f32, ht->s32d, e->grid_long[blk ? 1 : 0][R == 8 ? 1 : 0], pl->side->s[0]);
       if (err != cudaSuccess) return cuda_fail(err, "long-read tier launch");
       ++n;
-      VD_CUDA(cudaEventRecord(pl->ev_join, pl->side));
+      VD_CUDA(cudaEventRecord(pl->side->join[0], pl->side->s[0]));
     }
     // two-read items, on their own kernels (FP32 semiglobal only): 6-8 rows
-    // per lane, then up to 5
+    // per lane, and up to 5
     for (int k = 0; k < 2; ++k) {
       const int64_t lo = k ? nw : 0, hi = k ? np : nw;
       if (hi <= lo) continue;
@@ -1126,20 +1156,24 @@ int enqueue_tiers(vd_plan* pl, int* launches, bool capturing = false) {
       qp.n_items = hi - lo;
       qp.head = cnt + 6 + k;
       const int split = pl->chunk.pair_split;
+      const bool aside = k == 1 && narrow_aside;
+      if (aside) VD_CUDA(cudaStreamWaitEvent(pl->side->s[1], pl->side->fork, 0));
       err = launch_pair_f32(k == 0, split, bv, qp, &dt->f32, ht->s32, e->grid_pair[split == 7][k == 0 ? 1 : 0],
-                            pl->stream);
+                            aside ? pl->side->s[1] : pl->stream);
       if (err != cudaSuccess) return cuda_fail(err, "two-read tier launch");
+      if (aside) VD_CUDA(cudaEventRecord(pl->side->join[1], pl->side->s[1]));
       ++n;
     }
     q.items = (const WorkItem*)(d + L.o_items) + np + nl;
-    q.n_items = (long long)(pl->chunk.items.size() - np - nl);
+    q.n_items = (long long)ns;
     if (q.n_items > 0) {
       err = f64 ? launch_f64(anch, bv, q, &dt->f64, ht->s64, 1, e->grid[1][anch], pl->stream)
                 : launch_f32(anch, bv, q, &dt->f32, ht->s32, 0, e->grid[0][anch], pl->stream);
       if (err != cudaSuccess) return cuda_fail(err, "primary tier launch");
       ++n;
     }
-    if (nl > 0) VD_CUDA(cudaStreamWaitEvent(pl->stream, pl->ev_join, 0));
+    if (nl > 0) VD_CUDA(cudaStreamWaitEvent(pl->stream, pl->side->join[0], 0));
+    if (narrow_aside) VD_CUDA(cudaStreamWaitEvent(pl->stream, pl->side->join[1], 0));
     VD_CUDA(cudaEventRecordWithFlags(pl->ev_mid, pl->stream, evflags));
     BatchView rv = bv;
     rv.hap_sel = nullptr;
@@ -1364,23 +1398,19 @@ int vd_engine_create(int device, int64_t memory_mb, vd_engine** out) {
   std::snprintf(e->name, sizeof(e->name), "%s", prop.name);
   e->budget = (size_t)memory_mb << 20;
   int rc = VD_OK;
-  if ((err = cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking)) != cudaSuccess ||
+  if ((err = cudaStreamCreateWithPriority(&e->stream, cudaStreamNonBlocking, kOwnPriority)) != cudaSuccess ||
       (err = cudaEventCreate(&e->ev_begin)) != cudaSuccess || (err = cudaEventCreate(&e->ev_mid)) != cudaSuccess ||
       (err = cudaEventCreate(&e->ev_end)) != cudaSuccess ||
-      (err = cudaStreamCreateWithFlags(&e->side, cudaStreamNonBlocking)) != cudaSuccess ||
-      (err = cudaEventCreateWithFlags(&e->ev_fork, cudaEventDisableTiming)) != cudaSuccess ||
-      (err = cudaEventCreateWithFlags(&e->ev_join, cudaEventDisableTiming)) != cudaSuccess ||
+      (err = e->side.create()) != cudaSuccess ||
       (err = cudaMallocHost((void**)&e->htab, sizeof(TableSet))) != cudaSuccess) {
     rc = cuda_fail(err, "engine setup");
   }
   for (int k = 0; k < 2 && !rc; ++k) {
     vd_engine::Slot& sl = e->slots[k];
-    if ((err = cudaStreamCreateWithFlags(&sl.stream, cudaStreamNonBlocking)) != cudaSuccess ||
+    if ((err = cudaStreamCreateWithPriority(&sl.stream, cudaStreamNonBlocking, kOwnPriority)) != cudaSuccess ||
         (err = cudaEventCreate(&sl.ev[0])) != cudaSuccess || (err = cudaEventCreate(&sl.ev[1])) != cudaSuccess ||
         (err = cudaEventCreate(&sl.ev[2])) != cudaSuccess ||
-        (err = cudaStreamCreateWithFlags(&sl.side, cudaStreamNonBlocking)) != cudaSuccess ||
-        (err = cudaEventCreateWithFlags(&sl.fork, cudaEventDisableTiming)) != cudaSuccess ||
-        (err = cudaEventCreateWithFlags(&sl.join, cudaEventDisableTiming)) != cudaSuccess ||
+        (err = sl.side.create()) != cudaSuccess ||
         (err = cudaMallocHost((void**)&sl.hcnt, 16 * sizeof(unsigned long long))) != cudaSuccess)
       rc = cuda_fail(err, "engine pipeline setup");
   }
@@ -1395,7 +1425,7 @@ int vd_engine_destroy(vd_engine* e) {
   {
     DeviceGuard guard(e->device);
     if (e->stream) cudaStreamSynchronize(e->stream);
-    if (e->side) cudaStreamSynchronize(e->side);
+    e->side.synchronize();
     // plans still alive become empty shells; vd_plan_destroy frees the shell
     for (vd_plan* pl : e->plans) {
       if (pl->graph) cudaGraphExecDestroy(pl->graph);
@@ -1407,15 +1437,13 @@ int vd_engine_destroy(vd_engine* e) {
     e->plans.clear();
     for (vd_engine::Slot& sl : e->slots) {
       if (sl.stream) cudaStreamSynchronize(sl.stream);
-      if (sl.side) cudaStreamSynchronize(sl.side);
+      sl.side.synchronize();
       delete sl.pl;
       sl.pl = nullptr;
       sl.arena.release();
       for (cudaEvent_t& ev : sl.ev) if (ev) cudaEventDestroy(ev);
-      if (sl.fork) cudaEventDestroy(sl.fork);
-      if (sl.join) cudaEventDestroy(sl.join);
       if (sl.hcnt) cudaFreeHost(sl.hcnt);
-      if (sl.side) cudaStreamDestroy(sl.side);
+      sl.side.destroy();
       if (sl.stream) cudaStreamDestroy(sl.stream);
     }
     e->arena.release();
@@ -1426,9 +1454,7 @@ int vd_engine_destroy(vd_engine* e) {
     if (e->ev_begin) cudaEventDestroy(e->ev_begin);
     if (e->ev_mid) cudaEventDestroy(e->ev_mid);
     if (e->ev_end) cudaEventDestroy(e->ev_end);
-    if (e->ev_fork) cudaEventDestroy(e->ev_fork);
-    if (e->ev_join) cudaEventDestroy(e->ev_join);
-    if (e->side) cudaStreamDestroy(e->side);
+    e->side.destroy();
     if (e->stream) cudaStreamDestroy(e->stream);
   }
   if (e == g_default) g_default = nullptr;
@@ -1626,9 +1652,7 @@ int vd_forward(vd_engine* e, const vd_batch* b, const vd_params* p, double* out,
     pl.ev_begin = sl.ev[0];
     pl.ev_mid = sl.ev[1];
     pl.ev_end = sl.ev[2];
-    pl.side = sl.side;
-    pl.ev_fork = sl.fork;
-    pl.ev_join = sl.join;
+    pl.side = &sl.side;
     const double th = now_ms();
     const bool plain = p->schedule == VD_SCHEDULE_PLAIN;
     const BuildOpts& bo = lbo;
@@ -1690,9 +1714,7 @@ int vd_plan_create(vd_engine* e, const vd_batch* b, const vd_params* p, vd_plan*
   pl->ev_begin = e->ev_begin;
   pl->ev_mid = e->ev_mid;
   pl->ev_end = e->ev_end;
-  pl->side = e->side;
-  pl->ev_fork = e->ev_fork;
-  pl->ev_join = e->ev_join;
+  pl->side = &e->side;
   if (p->quality_offsets) {
     pl->has_offsets = true;
     for (int i = 0; i < 4; ++i) pl->offsets[i] = p->quality_offsets[i];

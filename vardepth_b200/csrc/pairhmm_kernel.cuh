@@ -958,6 +958,9 @@ template <typename T, bool ANCH>
 __global__ void __launch_bounds__(kWarpsPerBlock * kWarp, MinBlocks<T>::value)
 pairhmm_kernel(const __grid_constant__ BatchView bv, const __grid_constant__ QueueView qv,
                const Tables<T>* __restrict__ gtab, const __grid_constant__ Scalars<T> sc, const int tier) {
+  // an empty rescue list ends here (before the tables are staged: 19 -> 11 us for
+  // the three empty tiers of a small call)
+  if (qv.items == nullptr && *qv.count == 0) return;
   __shared__ Tables<T> tab;
   {
     const int words = (int)(sizeof(Tables<T>) / sizeof(int));
@@ -1070,6 +1073,7 @@ template <int kBlocks>
 __global__ void __launch_bounds__(kWarpsPerBlock * kWarp, kBlocks)
 pairhmm_drift_kernel(const __grid_constant__ BatchView bv, const __grid_constant__ QueueView qv,
                      const Tables<float>* __restrict__ gtab, const __grid_constant__ Scalars<float> sc) {
+  if (*qv.count == 0) return;
   __shared__ Tables<float> tab;
   {
     const int words = (int)(sizeof(Tables<float>) / sizeof(int));
