@@ -1698,6 +1698,48 @@ int vd_forward(vd_engine* e, const vd_batch* b, const vd_params* p, double* out,
   return VD_OK;
 }
 
+namespace {
+// The whole batch as one chunk in a slot (ignoring the memory budget), its tiers
+// and the copy of their counters enqueued on the slot's stream.  The engine's lock
+// is held and the slot is idle.
+int enqueue_whole(vd_engine* e, const vd_batch* b, const vd_params* p, vd_engine::Slot& sl, vd_stats* s) {
+  int rc = ensure_tables(e, p);
+  if (rc) return rc;
+  if (!sl.pl) sl.pl = new vd_plan();
+  vd_plan& pl = *sl.pl;
+  pl.chunk = HostChunk();
+  pl.eng = e;
+  pl.params = *p;
+  pl.stream = sl.stream;
+  pl.ev_begin = sl.ev[0];
+  pl.ev_mid = sl.ev[1];
+  pl.ev_end = sl.ev[2];
+  pl.side = &sl.side;
+  const double th = now_ms();
+  BuildOpts bo = build_opts(e);
+  bo.item_limit = batch_item_limit(e, b, p);
+  build_region_chunk(b, 0, b->n_regions, e->htab, p->quality_offsets != nullptr, p->anchored != 0,
+                     p->precision == VD_PRECISION_MIXED, pl.chunk, p->schedule == VD_SCHEDULE_PLAIN, bo);
+  HostChunk& c = pl.chunk;
+  pl.L = layout_for(c, b, max_grid_warps(e), long_warps(e, c));
+  s->host_ms += now_ms() - th;
+  if ((rc = sl.arena.reserve(pl.L.total))) return rc;
+  pl.base = (char*)sl.arena.p;
+  if ((rc = upload_chunk(&pl, b, &s->h2d_bytes))) return rc;
+  int launches = 0;
+  if ((rc = enqueue_tiers(&pl, &launches))) return rc;
+  if ((rc = enqueue_counter_read(&pl, sl.hcnt))) return rc;
+  s->pairs = c.n_out;
+  s->dp_cells = c.cells;
+  s->shared_cells = c.shared_cells;
+  s->work_items = (int64_t)c.items.size();
+  s->batches = 1;
+  s->kernel_launches = launches;
+  s->live_bytes = (int64_t)pl.L.total;
+  return VD_OK;
+}
+}  // namespace
+
 int vd_plan_create(vd_engine* e, const vd_batch* b, const vd_params* p, vd_plan** out) {
   if (!e || !out) return fail(VD_EINVAL, "engine or out is NULL");
   *out = nullptr;
@@ -2042,13 +2084,24 @@ int vd_region_genotypes(vd_engine* e, const vd_batch* b, const vd_params* p, con
   if (gl_off[G] > 0 && !out_gl) return fail(VD_EINVAL, "out_gl is NULL");
   const bool guard = opt->near_tie_guard == 1 && p->precision != VD_PRECISION_FLOAT64;
   std::vector<int> flags((size_t)G, 0);
-  vd_plan* pl = nullptr;
-  if ((rc = vd_plan_create(e, b, p, &pl))) return rc;
   vd_stats s{};
-  if ((rc = vd_plan_run(pl, &s))) { vd_plan_destroy(pl); return rc; }
   {
     std::lock_guard<std::mutex> lk(e->mu);
     DeviceGuard dguard(e->device);
+    // the forward pass as one chunk in a pipeline slot (its buffers stay with the
+    // engine; a plan would allocate, capture and free them on every call), the
+    // rest behind it on the slot's stream
+    vd_engine::Slot& sl = e->slots[0];
+    struct Drain {
+      vd_engine* e;
+      vd_engine::Slot& sl;
+      ~Drain() {
+        cudaStreamSynchronize(sl.stream);
+        if (sl.arena.bytes > e->budget) sl.arena.release();  // (this call ignores the memory budget)
+      }
+    } drain{e, sl};
+    if ((rc = enqueue_whole(e, b, p, sl, &s))) return rc;
+    vd_plan* pl = sl.pl;
     size_t off = 0;
     auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + std::max<size_t>(bytes, 1), 256); return o; };
     const size_t o_roff = take(n_rows * 8), o_rh = take(n_rows * 4), o_mq = take(n_rows * 8),
@@ -2057,7 +2110,7 @@ int vd_region_genotypes(vd_engine* e, const vd_batch* b, const vd_params* p, con
                  o_gl = take(gl_off[G] * 8), o_acc = take(acc_off[G] * 8), o_flag = take(G * 4);
     rc = e->geno_arena.reserve(off);
     char* d = (char*)e->geno_arena.p;
-    cudaStream_t sm = e->stream;
+    cudaStream_t sm = sl.stream;
     auto put = [&](size_t o, const void* src, size_t n) -> int {
       if (n) VD_CUDA(cudaMemcpyAsync(d + o, src, n, cudaMemcpyHostToDevice, sm));
       return VD_OK;
@@ -2098,7 +2151,9 @@ int vd_region_genotypes(vd_engine* e, const vd_batch* b, const vd_params* p, con
       if (err == cudaSuccess) err = cudaEventElapsedTime(&ms, e->ev_begin, e->ev_end);
       if (err != cudaSuccess) {
         rc = cuda_fail(err, "genotype post-processing");
-      } else {
+      } else if (!(rc = check_counters(pl, sl.hcnt, &s.rescued_fp32, &s.rescued_fp64, &s.rescued_robust,
+                                       &s.long_strip_runs, &s.long_strips)) &&
+                 !(rc = tier_times(pl, &s.kernel_ms, &s.primary_ms, &s.rescue_ms))) {
         if (out_certainty)
           for (int64_t k = 0; k < n_rows; ++k) out_certainty[row_read[k]] = cert[(size_t)k];
         s.kernel_ms += ms;
@@ -2108,7 +2163,6 @@ int vd_region_genotypes(vd_engine* e, const vd_batch* b, const vd_params* p, con
       }
     }
   }
-  vd_plan_destroy(pl);
   if (rc) return rc;
   if (out_guarded) for (int64_t g = 0; g < G; ++g) out_guarded[g] = flags[(size_t)g];
 
