@@ -495,4 +495,372 @@ pairhmm_grad_kernel(const __grid_constant__ BatchView bv, const __grid_constant_
   }
 }
 
+
+// ---- two pairs per warp (FP32, semiglobal, one-sided emission, sqrt-L) ----------
+// Two pairs with the same rows per lane go through grad_pair's passes together,
+// packed as float2 (x: first pair, y: second): one issue slot serves both in the
+// FMAs, and the shuffles, the buffer accesses and the step's bookkeeping are
+// shared.  Every element goes through grad_pair's operations in grad_pair's
+// order, so a pair's result is the same bits on either kernel (and under
+// VD_CHECKPOINT_ALL, which runs there).  The rows keep W = om of the next column
+// in place of mu and om, as the forward's two-read kernels do.  A half whose
+// haplotype is the shorter one sees only zeros from below past its end, which add
+// nothing to its sums.  What bounds it: FMA issue and the vertical chains at 8 to
+// 12 warps per SM (24 registers a row).  40 regions, 3.9e9 cells: 14.7 -> 9.4 ms;
+// 4,000 pairs of 100 / 150 / 250 bases x 400: 1.08 / 1.20 / 1.42 -> 0.62 / 0.69 / 1.10 ms.
+template <int R, int SUB>
+__device__ __forceinline__ void grad_pair2(const BatchView& bv, const GradView& gv, const RescueEntry ia,
+                                           const RescueEntry ib, const Tables<float>* __restrict__ tb,
+                                           const Scalars<float>& sc, const GradTables* __restrict__ gt,
+                                           const GradScalars& gs, const int lane, float* __restrict__ slot,
+                                           float2* __restrict__ sbuf) {
+  constexpr unsigned FULL = 0xffffffffu;
+  const int64_t roa = bv.read_off[ia.read], rob = bv.read_off[ib.read];
+  const int na = (int)(bv.read_off[ia.read + 1] - roa), nb = (int)(bv.read_off[ib.read + 1] - rob);
+  const uint8_t* __restrict__ qa = bv.read_quals + roa;
+  const uint8_t* __restrict__ qb = bv.read_quals + rob;
+  const int64_t hoa = bv.hap_off[ia.hap], hob = bv.hap_off[ib.hap];
+  const int ma = (int)(bv.hap_off[ia.hap + 1] - hoa), mb = (int)(bv.hap_off[ib.hap + 1] - hob);
+  const uint8_t* __restrict__ ha = bv.hap_bases + hoa - 1;  // ha[j] = base of column j >= 1
+  const uint8_t* __restrict__ hb = bv.hap_bases + hob - 1;
+  const int M = max(ma, mb);
+  const int steps = grad_steps(M);
+  const int C = grad_interval(steps, false);
+  const int nseg = (steps + C - 1) / C;
+  // a sub-segment's steps are unrolled for the fewest rows only (at 8 rows that
+  // spills 2.8 KB: 4,000 pairs of 250 bases 1.10 -> 1.78 ms; at 1 row 0.33 -> 0.29)
+  constexpr int kUnrollSub = R <= 2 ? SUB : 1, kUnrollRun = 4;
+  constexpr int CKW = 2 * R + 2;  // checkpoint words (float2) per lane
+  constexpr int BFW = 2 * R + 1;  // buffer words (float2) per lane and step
+  float2* __restrict__ ck = reinterpret_cast<float2*>(slot);
+  float2* __restrict__ sub = ck + (long long)nseg * CKW * kWarp;
+
+  const float2 k2 = make_float2(sc.k2, sc.k2), x = make_float2(sc.x, sc.x), c2 = make_float2(sc.c, sc.c);
+  const bool lane0 = lane == 0, lane31 = lane == kWarp - 1;
+  PairRows<R> rw;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const int i = lane * R + r;
+    const unsigned q0 = i < na ? qa[i] : 0u, q1 = i < nb ? qb[i] : 0u;
+    rw.ra[r] = i < na ? (uint32_t)bv.read_bases[roa + i] : kNeverBase;
+    rw.rb[r] = i < nb ? (uint32_t)bv.read_bases[rob + i] : kNeverBase;
+    rw.miss[r] = make_float2(i < na ? tb->miss[q0] : 0.f, i < nb ? tb->miss[q1] : 0.f);
+    rw.K[r] = make_float2(i < na ? tb->K[q0] : 0.f, i < nb ? tb->K[q1] : 0.f);
+    rw.X[r] = make_float2(i < na ? (i == na - 1 ? tb->A[q0] : tb->X[q0]) : 1.f,
+                          i < nb ? (i == nb - 1 ? tb->A[q1] : tb->X[q1]) : 1.f);
+    rw.W[r] = make_float2(0.f, 0.f);
+    rw.s[r] = make_float2(0.f, 0.f);
+  }
+  float2 s_top = make_float2(0.f, 0.f), u_bot = make_float2(0.f, 0.f);
+  double acc_a = 0.0, acc_b = 0.0;
+
+  // one forward step; INNER: every lane at a column in 1 .. min(ma, mb); REC: the
+  // lane's column values go to e (mu, om per row, u handed in); SUM: lane 31 sums its
+  // bottom row
+  auto fstep = [&](auto inner_tag, auto rec_tag, auto sum_tag, const int t, float2* __restrict__ e) {
+    constexpr bool INNER = decltype(inner_tag)::value, REC = decltype(rec_tag)::value;
+    const int j = t - lane;
+    uint32_t b0, b1;
+    if (INNER) {
+      b0 = __ldg(ha + j);
+      b1 = __ldg(hb + j);
+    } else {
+      b0 = j > 0 && j <= ma ? (uint32_t)__ldg(ha + j) : 0u;
+      b1 = j > 0 && j <= mb ? (uint32_t)__ldg(hb + j) : 0u;
+    }
+    float2 u_in = shfl_up2(u_bot);
+    float2 s_in = shfl_up2(rw.s[R - 1]);
+    u_in = lane0 ? c2 : u_in;
+    s_in = lane0 ? c2 : s_in;
+    if (!INNER && j == 0) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        rw.W[r] = make_float2(0.f, 0.f);
+        rw.s[r] = make_float2(0.f, 0.f);
+      }
+      s_top = make_float2(0.f, 0.f);
+    }
+    const bool rec = REC && (INNER || (unsigned)j <= (unsigned)M);
+    float2 s_above = s_top, nu = u_in;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      float2 mu = s_above;
+      mul_if_ne(mu.x, rw.ra[r], b0, rw.miss[r].x);
+      mul_if_ne(mu.y, rw.rb[r], b1, rw.miss[r].y);
+      const float2 om = rw.W[r];
+      if (rec) {
+        e[r * kWarp] = mu;
+        e[(R + r) * kWarp] = om;
+      }
+      const float2 un = __ffma2_rn(rw.X[r], nu, mu);
+      const float2 sn = __ffma2_rn(k2, om, __ffma2_rn(rw.K[r], nu, mu));
+      s_above = rw.s[r];
+      rw.W[r] = __ffma2_rn(x, om, mu);
+      rw.s[r] = sn;
+      nu = un;
+    }
+    if (rec) e[2 * R * kWarp] = u_in;
+    u_bot = nu;
+    s_top = s_in;
+    if (decltype(sum_tag)::value && (INNER || (lane31 && j >= 0))) {
+      if (INNER || j <= ma) acc_a += (double)u_bot.x;
+      if (INNER || j <= mb) acc_b += (double)u_bot.y;
+    }
+  };
+  // forward steps [ta, tz) without a record
+  auto run = [&](auto sum_tag, const int ta, const int tz) {
+    int t = ta;
+    for (; t < tz && t < kWarp; ++t) fstep(std::false_type{}, std::false_type{}, sum_tag, t, nullptr);
+    const int ti = min(tz, min(ma, mb) + 1);
+#pragma unroll kUnrollRun
+    for (; t < ti; ++t) fstep(std::true_type{}, std::false_type{}, sum_tag, t, nullptr);
+    for (; t < tz; ++t) fstep(std::false_type{}, std::false_type{}, sum_tag, t, nullptr);
+  };
+  auto save_state = [&](float2* __restrict__ area, const int k) {
+    float2* e = area + (long long)k * CKW * kWarp + lane;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      e[r * kWarp] = rw.W[r];
+      e[(R + r) * kWarp] = rw.s[r];
+    }
+    e[2 * R * kWarp] = s_top;
+    e[(2 * R + 1) * kWarp] = u_bot;
+  };
+  auto load_state = [&](const float2* __restrict__ area, const int k) {
+    const float2* e = area + (long long)k * CKW * kWarp + lane;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      rw.W[r] = e[r * kWarp];
+      rw.s[r] = e[(R + r) * kWarp];
+    }
+    s_top = e[2 * R * kWarp];
+    u_bot = e[(2 * R + 1) * kWarp];
+  };
+
+  // ---- first forward pass ----
+  for (int k = 0; k < nseg; ++k) {
+    save_state(ck, k);
+    const int t1 = min(steps, (k + 1) * C);
+    run(std::true_type{}, k * C, t1);
+  }
+  const double Za = __shfl_sync(FULL, acc_a, kWarp - 1), Zb = __shfl_sync(FULL, acc_b, kWarp - 1);
+  double lna = 0.0, lnb = 0.0;
+  for (int i = lane; i < na; i += kWarp) lna += tb->lnN[qa[i]];
+  for (int i = lane; i < nb; i += kWarp) lnb += tb->lnN[qb[i]];
+#pragma unroll
+  for (int s = 16; s; s >>= 1) {
+    lna += __shfl_xor_sync(FULL, lna, s);
+    lnb += __shfl_xor_sync(FULL, lnb, s);
+  }
+  const bool oka = Za >= (double)sc.final_floor && Za < HUGE_VAL, okb = Zb >= (double)sc.final_floor && Zb < HUGE_VAL;
+  // a half that left the FP32 range goes to the FP64 pass
+  auto hand_on = [&](const RescueEntry& item) {
+    if (lane == 0) {
+      const double nan = __longlong_as_double(0x7ff8000000000000LL);
+      gv.out_ln[item.out] = nan;
+      for (int k = 0; k < 6; ++k) gv.out_jac[item.out * 6 + k] = nan;
+      const unsigned long long s = atomicAdd(gv.spill_count, 1ull);
+      if ((long long)s < gv.spill_cap) gv.spill[s] = item;
+      else atomicOr(gv.error_flag, 1);
+    }
+  };
+  if (!oka) hand_on(ia);
+  if (!okb && ib.out >= 0) hand_on(ib);
+  __syncwarp();
+  if (!oka && !okb) return;
+
+  // ---- reverse sweep ----
+  auto rho_exp = [&](double Z, bool ok) {
+    return ok ? min(GradConsts<float>::kMax, GradConsts<float>::kTarget - ilogb(Z)) : -126;
+  };
+  const int ra2 = rho_exp(Za, oka), rb2 = rho_exp(Zb, okb);
+  // (a half handed on runs along from 0: nothing of it is used)
+  const float2 rho = make_float2(oka ? pow2T(ra2, 0.f) : 0.f, okb ? pow2T(rb2, 0.f) : 0.f);
+  float2 ome[R], ups[R], pu[R], ps[R], bM[R];
+  const float2 zero = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int r = 0; r < R; ++r) ome[r] = ups[r] = pu[r] = ps[r] = bM[r] = zero;
+  float2 Bk2 = zero, Ax = zero, top_u = zero, top_s = zero, pend_s = zero;
+
+  auto bstep = [&](auto inner_tag, const int t, const float2* __restrict__ e) {
+    constexpr bool INNER = decltype(inner_tag)::value;
+    const int j = t - lane;
+    float2 in_u = make_float2(__shfl_down_sync(FULL, top_u.x, 1), __shfl_down_sync(FULL, top_u.y, 1));
+    float2 in_s_next = make_float2(__shfl_down_sync(FULL, top_s.x, 1), __shfl_down_sync(FULL, top_s.y, 1));
+    if (lane31) {
+      in_u = make_float2(INNER || (unsigned)j <= (unsigned)ma ? rho.x : 0.f,
+                         INNER || (unsigned)j <= (unsigned)mb ? rho.y : 0.f);
+      in_s_next = zero;
+    }
+    const float2 in_s = pend_s;
+    pend_s = in_s_next;
+    uint32_t b0, b1;
+    if (INNER) {
+      b0 = __ldg(ha + j);
+      b1 = __ldg(hb + j);
+    } else {
+      if ((unsigned)j > (unsigned)M) {
+        top_u = zero;
+        top_s = zero;
+        return;
+      }
+      b0 = j > 0 && j <= ma ? (uint32_t)__ldg(ha + j) : 0u;
+      b1 = j > 0 && j <= mb ? (uint32_t)__ldg(hb + j) : 0u;
+    }
+    float2 muf[R], nu[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) muf[r] = e[r * kWarp];
+    nu[0] = e[2 * R * kWarp];
+#pragma unroll
+    for (int r = 1; r < R; ++r) nu[r] = __ffma2_rn(rw.X[r - 1], nu[r - 1], muf[r - 1]);
+    float2 cu = in_u, cs = in_s;
+#pragma unroll
+    for (int r = R - 1; r >= 0; --r) {
+      const float2 sb = cs, ub = cu;
+      const float2 omf = e[(R + r) * kWarp];
+      const float2 omb = __ffma2_rn(x, ome[r], __fmul2_rn(k2, sb));
+      const float2 mub = __fadd2_rn(__fadd2_rn(ub, sb), ome[r]);
+      pu[r] = __ffma2_rn(ub, nu[r], pu[r]);
+      ps[r] = __ffma2_rn(sb, nu[r], ps[r]);
+      // (a matching cell adds nothing to bM and keeps mub)
+      float2 up = mub;
+      if (rw.ra[r] != b0) { bM[r].x = __fmaf_rn(mub.x, muf[r].x, bM[r].x); up.x = mub.x * rw.miss[r].x; }
+      if (rw.rb[r] != b1) { bM[r].y = __fmaf_rn(mub.y, muf[r].y, bM[r].y); up.y = mub.y * rw.miss[r].y; }
+      Bk2 = __ffma2_rn(sb, omf, Bk2);
+      Ax = __ffma2_rn(ome[r], omf, Ax);
+      ome[r] = omb;
+      cu = __ffma2_rn(rw.X[r], ub, __fmul2_rn(rw.K[r], sb));
+      cs = ups[r];
+      ups[r] = up;
+    }
+    top_u = cu;
+    top_s = ups[0];
+  };
+
+  for (int k = nseg - 1; k >= 0; --k) {
+    const int t0 = k * C;
+    const int t1 = min(steps, t0 + C);
+    load_state(ck, k);
+    const int nsub = (t1 - t0 + SUB - 1) / SUB;
+    for (int q = 0; q + 1 < nsub; ++q) {
+      save_state(sub, q);
+      run(std::false_type{}, t0 + q * SUB, t0 + (q + 1) * SUB);
+    }
+    for (int q = nsub - 1; q >= 0; --q) {
+      const int ta = t0 + q * SUB;
+      const int tz = min(t1, ta + SUB);
+      if (q + 1 != nsub) load_state(sub, q);  // (the last one's state is at hand)
+      // each lane reads back what it wrote itself
+      if (tz - ta == SUB && ta >= kWarp && tz - 1 <= min(ma, mb)) {
+#pragma unroll kUnrollSub
+        for (int u = 0; u < SUB; ++u)
+          fstep(std::true_type{}, std::true_type{}, std::false_type{}, ta + u, sbuf + u * BFW * kWarp + lane);
+#pragma unroll kUnrollSub
+        for (int u = SUB - 1; u >= 0; --u) bstep(std::true_type{}, ta + u, sbuf + u * BFW * kWarp + lane);
+      } else {
+        for (int t = ta; t < tz; ++t)
+          fstep(std::false_type{}, std::true_type{}, std::false_type{}, t, sbuf + (t - ta) * BFW * kWarp + lane);
+        for (int t = tz - 1; t >= ta; --t) bstep(std::false_type{}, t, sbuf + (t - ta) * BFW * kWarp + lane);
+      }
+    }
+  }
+
+  // ---- chain rule to theta (FP64), as in grad_pair ----
+  auto finish = [&](const RescueEntry& item, int n, int m, const uint8_t* rq, double Z, int rho_log2, double lnN,
+                    auto half) {
+    const double inv = 1.0 / (ldexp(1.0, rho_log2) * Z);
+    double jg = 0.0, jx = 0.0, jo0 = 0.0, jo1 = 0.0, jo2 = 0.0, jo3 = 0.0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const int i = lane * R + r;
+      if (i < n) {
+        const unsigned q = rq[i];
+        const bool last = i == n - 1;
+        const double bX = (double)half(rw.X[r]) * (double)half(pu[r]);
+        const double bK = (double)half(rw.K[r]) * (double)half(ps[r]);
+        jg += (bX * (last ? gs.dlnA_g : gs.dlnX_g) + bK * gs.dlnK_g) * inv + gs.dlnN_g;
+        jx += (bX * (last ? 0.0 : gs.dlnX_x) + bK * gs.dlnK_x) * inv;
+        const double d = ((double)half(bM[r]) * gt->dlnmiss[q] + 0.0 * gt->dlnhit[q] - (bX + bK) * gt->dlnN[q]) * inv +
+                         gt->dlnN[q];
+        const int b = gt->bin[q];
+        jo0 += b == 0 ? d : 0.0;
+        jo1 += b == 1 ? d : 0.0;
+        jo2 += b == 2 ? d : 0.0;
+        jo3 += b == 3 ? d : 0.0;
+      }
+    }
+    jg += (double)half(k2) * (double)half(Bk2) * gs.dlnk2_g * inv;
+    jx += ((double)half(k2) * (double)half(Bk2) * gs.dlnk2_x + (double)half(Ax) * gs.dx_x) * inv;
+#pragma unroll
+    for (int s = 16; s; s >>= 1) {
+      jg += __shfl_xor_sync(FULL, jg, s);
+      jx += __shfl_xor_sync(FULL, jx, s);
+      jo0 += __shfl_xor_sync(FULL, jo0, s);
+      jo1 += __shfl_xor_sync(FULL, jo1, s);
+      jo2 += __shfl_xor_sync(FULL, jo2, s);
+      jo3 += __shfl_xor_sync(FULL, jo3, s);
+    }
+    if (lane == 0) {
+      gv.out_ln[item.out] = log(Z) - ((double)sc.ln_c + log((double)(m + 1))) + lnN;
+      double* J = gv.out_jac + item.out * 6;
+      J[0] = jg;
+      J[1] = jx;
+      J[2] = jo0;
+      J[3] = jo1;
+      J[4] = jo2;
+      J[5] = jo3;
+    }
+  };
+  if (oka) finish(ia, na, ma, qa, Za, ra2, lna, [](const float2 v) { return v.x; });
+  if (okb && ib.out >= 0) finish(ib, nb, mb, qb, Zb, rb2, lnb, [](const float2 v) { return v.y; });
+  __syncwarp();
+}
+
+// Shared memory of one warp's sub-segment buffer.
+constexpr int grad_pair_smem_per_warp(int max_R, int sub) { return sub * (2 * max_R + 1) * kWarp * (int)sizeof(float2); }
+
+// Persistent kernel of the two-pair items: entries 2i and 2i + 1 of the list are
+// one item (the second may be a filler, out = -1).  Rows take 24 registers each:
+// 5-8 of them run 2 blocks per SM, up to 4 run 3.
+template <int kLoR, int kHiR, int kSteps, int kBlocks>
+__global__ void __launch_bounds__(kWarpsPerBlock * kWarp, kBlocks)
+pairhmm_grad_pair_kernel(const __grid_constant__ BatchView bv, const __grid_constant__ GradView gv,
+                         const Tables<float>* __restrict__ gtab, const __grid_constant__ Scalars<float> sc,
+                         const GradTables* __restrict__ gtt, const __grid_constant__ GradScalars gs) {
+  __shared__ Tables<float> tab;
+  __shared__ GradTables gt;
+  {
+    const int words = (int)(sizeof(Tables<float>) / sizeof(int));
+    const int* src = reinterpret_cast<const int*>(gtab);
+    int* dst = reinterpret_cast<int*>(&tab);
+    for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
+    const int gwords = (int)(sizeof(GradTables) / sizeof(int));
+    const int* gsrc = reinterpret_cast<const int*>(gtt);
+    int* gdst = reinterpret_cast<int*>(&gt);
+    for (int i = threadIdx.x; i < gwords; i += blockDim.x) gdst[i] = gsrc[i];
+  }
+  __syncthreads();
+  extern __shared__ __align__(16) unsigned char grad_pair_dyn[];
+  const int lane = threadIdx.x & (kWarp - 1);
+  const long long gw = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
+  float* slot = reinterpret_cast<float*>(gv.scratch + gw * gv.slot_bytes);
+  float2* sbuf = reinterpret_cast<float2*>(grad_pair_dyn + (threadIdx.x >> 5) * grad_pair_smem_per_warp(kHiR, kSteps));
+  for (;;) {
+    unsigned long long i = 0;
+    if (lane == 0) i = atomicAdd(gv.head, 1ull);
+    i = __shfl_sync(0xffffffffu, i, 0);
+    if ((long long)i >= gv.n_items) break;
+    const RescueEntry ia = gv.items[2 * i], ib = gv.items[2 * i + 1];
+    switch (code_R(bv.read_code[ia.read])) {
+#define VD_GPCASE(r)                                                                                           \
+  case r:                                                                                                      \
+    if constexpr (r >= kLoR && r <= kHiR) grad_pair2<r, kSteps>(bv, gv, ia, ib, &tab, sc, &gt, gs, lane, slot, sbuf); \
+    break;
+      VD_GPCASE(1) VD_GPCASE(2) VD_GPCASE(3) VD_GPCASE(4) VD_GPCASE(5) VD_GPCASE(6) VD_GPCASE(7) VD_GPCASE(8)
+#undef VD_GPCASE
+      default: break;
+    }
+  }
+}
+
 }  // namespace vd

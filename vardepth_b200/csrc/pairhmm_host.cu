@@ -216,6 +216,7 @@ struct vd_engine {
   int grid_drift = 0;                 // blocks of the drift tier (no more than grid[0][0])
   int grid_long[2][2] = {{0, 0}, {0, 0}};  // blocks of the long-read kernels [block][R == 8] (<= grid[0][0])
   int grid_grad[2] = {0, 0};          // blocks of the gradient kernel [f64]
+  int grid_grad_pair[2] = {0, 0};     // blocks of the two-pair gradient kernels [wide]
   vd_tuning tuning{256, 0x1fe, 0, 0, VD_LONG_WARP, 6, kLongGroupMax, {0}};  // vd_engine_set_tuning
   DevBuf grad_arena;                  // inputs, lists and scratch of vd_forward_backward
   DevBuf geno_arena;                  // buffers of vd_region_genotypes
@@ -1307,6 +1308,10 @@ int init_engine_grids(vd_engine* e) {
     err = occupancy_grad(f != 0, &bps);
     if (err != cudaSuccess) return cuda_fail(err, "occupancy query");
     e->grid_grad[f] = std::max(1, bps) * e->sm_count;
+    bps = 0;
+    err = occupancy_grad_pair(f != 0, &bps);
+    if (err != cudaSuccess) return cuda_fail(err, "occupancy query");
+    e->grid_grad_pair[f] = std::max(1, bps) * e->sm_count;
   }
   return VD_OK;
 }
@@ -1924,19 +1929,46 @@ int vd_forward_backward(vd_engine* e, const vd_batch* b, const vd_params* p, int
       for (int64_t r = b->region_read_off[g]; r < b->region_read_off[g + 1]; ++r)
         for (int64_t h = b->region_hap_off[g]; h < b->region_hap_off[g + 1]; ++h) add(r, h, o++);
   }
-  // group by kernel variant, longest haplotype first inside a group
+  // group by kernel (two pairs per warp with 5-8 rows per lane, with up to 4, one
+  // pair) and variant, longest haplotype first inside a group
   auto hlen = [&](const RescueEntry& x) { return b->hap_off[x.hap + 1] - b->hap_off[x.hap]; };
-  std::stable_sort(items.begin(), items.end(), [&](const RescueEntry& x, const RescueEntry& y) {
-    const int cx = c.read_code[x.read] & 0x1ff, cy = c.read_code[y.read] & 0x1ff;
-    if (cx != cy) return cx > cy;
-    return hlen(x) > hlen(y);
-  });
+  const bool packed = !f64_only && !store_all && !p->anchored;
+  auto kernel_of = [&](int code) { return !packed || code_general(code) ? 2 : code_R(code) >= 5 ? 0 : 1; };
+  {
+    // (counting sort over kernel, code and length: the list is in region order)
+    const size_t n = items.size();
+    std::vector<std::pair<uint64_t, uint32_t>> key(n);
+    for (size_t k = 0; k < n; ++k) {
+      const int code = c.read_code[items[k].read] & 0x1ff;
+      key[k] = {((uint64_t)kernel_of(code) << 48) | ((uint64_t)(0x1ff - code) << 36) |
+                    ((1ull << 36) - 1 - (uint64_t)hlen(items[k])), (uint32_t)k};
+    }
+    std::stable_sort(key.begin(), key.end(), [](const auto& x, const auto& y) { return x.first < y.first; });
+    std::vector<RescueEntry> sorted;
+    sorted.reserve(n + 16);
+    for (size_t k = 0; k < n; ++k) {
+      sorted.push_back(items[key[k].second]);
+      // the last pair of a packed group with an odd count runs beside a copy of itself
+      const bool end = k + 1 == n || (key[k + 1].first >> 36) != (key[k].first >> 36);
+      if (end && (key[k].first >> 48) < 2 && (sorted.size() & 1)) {
+        sorted.push_back(sorted.back());
+        sorted.back().out = -1;
+      }
+    }
+    items.swap(sorted);
+  }
+  int64_t n_kernel[3] = {0, 0, 0};
+  for (const RescueEntry& x : items) ++n_kernel[kernel_of(c.read_code[x.read])];
   long long slot_bytes = 256;
   for (const RescueEntry& x : items)
     slot_bytes = std::max(slot_bytes, grad_slot_bytes(code_R(c.read_code[x.read]), (int)hlen(x), store_all));
   slot_bytes = (long long)align_up((size_t)slot_bytes, 256);
   const int grid32 = e->grid_grad[0], grid64 = e->grid_grad[1];
-  const int64_t slots = (int64_t)std::max(grid32, grid64) * kWarpsPerBlock;
+  // the two-pair kernels run side by side, each with its own slots; the others
+  // follow them and use the same
+  const int64_t slots_wide = n_kernel[0] ? (int64_t)e->grid_grad_pair[1] * kWarpsPerBlock : 0;
+  const int64_t slots_narrow = n_kernel[1] ? (int64_t)e->grid_grad_pair[0] * kWarpsPerBlock : 0;
+  const int64_t slots = std::max(slots_wide + slots_narrow, (int64_t)std::max(grid32, grid64) * kWarpsPerBlock);
 
   size_t off = 0;
   auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + std::max<size_t>(bytes, 1), 256); return o; };
@@ -1985,14 +2017,35 @@ int vd_forward_backward(vd_engine* e, const vd_batch* b, const vd_params* p, int
   cudaGetLastError();
   if (!items.empty()) {
     cudaError_t err;
-    if (!f64_only) {
-      gv.items = (const RescueEntry*)(d + o_items);
-      gv.count = nullptr;
-      gv.n_items = (long long)items.size();
+    gv.spill = (RescueEntry*)(d + o_spill);
+    gv.spill_count = cnt + 2;
+    gv.spill_cap = (long long)items.size();
+    gv.count = nullptr;
+    const bool aside = n_kernel[0] && n_kernel[1];
+    if (aside) {
+      VD_CUDA(cudaEventRecord(e->side.fork, st_));
+      VD_CUDA(cudaStreamWaitEvent(e->side.s[1], e->side.fork, 0));
+    }
+    for (int k = 0; k < 2; ++k) {
+      if (!n_kernel[k]) continue;
+      GradView gp = gv;
+      gp.items = (const RescueEntry*)(d + o_items) + (k ? n_kernel[0] : 0);
+      gp.n_items = n_kernel[k] / 2;
+      gp.head = cnt + (k ? 6 : 5);
+      gp.scratch = (char*)(d + o_scratch) + (k ? slots_wide * slot_bytes : 0);
+      err = launch_grad_pair_f32(k == 0, bv, gp, &dt->f32, ht->s32, (const GradTables*)(d + o_gt), gs,
+                                 e->grid_grad_pair[k == 0 ? 1 : 0], aside && k == 1 ? e->side.s[1] : st_);
+      if (err != cudaSuccess) return cuda_fail(err, "two-pair gradient launch");
+      ++s.kernel_launches;
+    }
+    if (aside) {
+      VD_CUDA(cudaEventRecord(e->side.join[1], e->side.s[1]));
+      VD_CUDA(cudaStreamWaitEvent(st_, e->side.join[1], 0));
+    }
+    if (!f64_only && n_kernel[2]) {
+      gv.items = (const RescueEntry*)(d + o_items) + n_kernel[0] + n_kernel[1];
+      gv.n_items = n_kernel[2];
       gv.head = cnt + 0;
-      gv.spill = (RescueEntry*)(d + o_spill);
-      gv.spill_count = cnt + 2;
-      gv.spill_cap = (long long)items.size();
       err = launch_grad_f32(bv, gv, &dt->f32, ht->s32, (const GradTables*)(d + o_gt), gs, grid32, st_);
       if (err != cudaSuccess) return cuda_fail(err, "gradient FP32 pass launch");
       ++s.kernel_launches;
@@ -2023,7 +2076,7 @@ int vd_forward_backward(vd_engine* e, const vd_batch* b, const vd_params* p, int
   s.kernel_ms = ms;
   const unsigned flags = (unsigned)(hc[4] & 0xffffffffu);
   if (flags & 1u) return fail(VD_EOVERFLOW, "gradient spill list overflow");
-  s.fp64_pairs = f64_only ? (int64_t)items.size() : (int64_t)hc[2];
+  s.fp64_pairs = f64_only ? n_kernel[2] : (int64_t)hc[2];
   for (int64_t o : empty_slots) {
     ln[(size_t)o] = -HUGE_VAL;
     for (int k = 0; k < 6; ++k) jac[(size_t)o * 6 + k] = 0.0;

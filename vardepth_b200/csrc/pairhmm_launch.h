@@ -35,6 +35,12 @@ cudaError_t launch_grad_f64(const BatchView& bv, const GradView& gv, const Table
                             const Scalars<double>& sc, const GradTables* gt, const GradScalars& gs, int grid,
                             cudaStream_t stream);
 cudaError_t occupancy_grad(bool fp64, int* blocks_per_sm);
+// two pairs per warp (FP32, semiglobal): rows 5-8 per lane (wide) or up to 4; the
+// list holds entries 2i, 2i + 1 per item, n_items of them
+cudaError_t launch_grad_pair_f32(bool wide, const BatchView& bv, const GradView& gv, const Tables<float>* tab,
+                                 const Scalars<float>& sc, const GradTables* gt, const GradScalars& gs, int grid,
+                                 cudaStream_t stream);
+cudaError_t occupancy_grad_pair(bool wide, int* blocks_per_sm);
 // bytes of one warp slot's checkpoints and segment buffer (sized for the FP64 pass)
 long long grad_slot_bytes(int R, int m, bool store_all);
 // region post-processing (pairhmm_genotype.cu)
