@@ -181,6 +181,8 @@ struct SideStreams {
   cudaStream_t s[2] = {nullptr, nullptr};
   cudaEvent_t fork = nullptr, join[2] = {nullptr, nullptr};
   cudaError_t create() {
+    if (join[1]) return cudaSuccess;
+    destroy();
     cudaError_t err = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
     for (int k = 0; k < 2 && err == cudaSuccess; ++k)
       if ((err = cudaStreamCreateWithPriority(&s[k], cudaStreamNonBlocking, kOwnPriority + (k ? 1 : -1))) ==
@@ -198,6 +200,10 @@ struct SideStreams {
     *this = SideStreams();
   }
 };
+
+// Inputs and lists of a chunk up to this size go to the device as one copy from
+// pinned memory instead of eight from the caller's (each a few us).
+constexpr size_t kStagingBytes = (size_t)256 << 10;
 
 // ---- engine -----------------------------------------------------------------------
 
@@ -238,10 +244,30 @@ struct vd_engine {
     SideStreams side;
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
     unsigned long long* hcnt = nullptr;  // pinned copy of the tier counters
+    char* staging = nullptr;             // pinned, kStagingBytes: the inputs of a small chunk
+    bool ready = false;
+    // the slot's streams, events and pinned memory, made when it is first used
+    // (the second slot only by batches of several chunks)
+    cudaError_t create() {
+      if (ready) return cudaSuccess;
+      cudaError_t err = cudaSuccess;
+      if (!stream) err = cudaStreamCreateWithPriority(&stream, cudaStreamNonBlocking, kOwnPriority);
+      for (int k = 0; k < 3 && err == cudaSuccess; ++k)
+        if (!ev[k]) err = cudaEventCreate(&ev[k]);
+      if (err == cudaSuccess) err = side.create();
+      if (err == cudaSuccess && !hcnt) {
+        void* p = nullptr;
+        err = cudaMallocHost(&p, 256 + kStagingBytes);
+        hcnt = (unsigned long long*)p;
+        staging = (char*)p + 256;
+      }
+      ready = err == cudaSuccess;
+      return err;
+    }
     std::vector<double> stage;           // pair-form outputs before the scatter
     vd_plan* pl = nullptr;
     bool busy = false;
-    int launches = 0;
+    bool deferred = false;               // its rescue tiers wait for the counters
   };
   Slot slots[2];
 };
@@ -1012,6 +1038,7 @@ struct vd_plan {
   bool has_offsets = false;
   cudaGraphExec_t graph = nullptr;
   int graph_launches = 0;  // kernels in the captured graph
+  bool filled = false;     // the upload filled the outputs with -inf (some pairs are empty)
   // stream and tier events the plan's work is enqueued on (the engine's own,
   // or a pipeline slot's in vd_forward)
   cudaStream_t stream = nullptr;
@@ -1039,16 +1066,18 @@ BatchView batch_view(vd_plan* pl) {
   return bv;
 }
 
-int upload_chunk(vd_plan* pl, const vd_batch* b, int64_t* h2d) {
-  vd_engine* e = pl->eng;
+int upload_chunk(vd_plan* pl, const vd_batch* b, int64_t* h2d, char* staging = nullptr) {
   HostChunk& c = pl->chunk;
   char* d = pl->base;
   const int64_t read_bytes = c.read_off.back();
   const int64_t hap_bytes = c.hap_off.back();
   int64_t bytes = 0;
+  const size_t inputs = pl->L.o_out;  // everything before the outputs is input
+  if (inputs > kStagingBytes) staging = nullptr;
   auto put = [&](size_t off, const void* src, size_t n) -> int {
     if (n == 0) return VD_OK;
-    VD_CUDA(cudaMemcpyAsync(d + off, src, n, cudaMemcpyHostToDevice, pl->stream));
+    if (staging) std::memcpy(staging + off, src, n);
+    else VD_CUDA(cudaMemcpyAsync(d + off, src, n, cudaMemcpyHostToDevice, pl->stream));
     bytes += (int64_t)n;
     return VD_OK;
   };
@@ -1065,7 +1094,10 @@ int upload_chunk(vd_plan* pl, const vd_batch* b, int64_t* h2d) {
   if ((rc = put(pl->L.o_hshare, c.hap_share.data(), c.hap_share.size() * sizeof(int32_t)))) return rc;
   if ((rc = put(pl->L.o_items, c.items.data(), c.items.size() * sizeof(WorkItem)))) return rc;
   if ((rc = put(pl->L.o_loff, c.long_off.data(), c.long_off.size() * sizeof(int64_t)))) return rc;
-  if (c.n_out > 0) {
+  if (staging) VD_CUDA(cudaMemcpyAsync(d, staging, inputs, cudaMemcpyHostToDevice, pl->stream));
+  // (the tiers write every pair that is not empty)
+  pl->filled = c.n_out > c.pairs_scored;
+  if (pl->filled) {
     fill_kernel<<<(int)std::min<int64_t>(4096, (c.n_out + 255) / 256), 256, 0, pl->stream>>>(
         (double*)(d + pl->L.o_out), c.n_out, -HUGE_VAL);
     VD_CUDA(cudaGetLastError());
@@ -1076,7 +1108,10 @@ int upload_chunk(vd_plan* pl, const vd_batch* b, int64_t* h2d) {
 
 // Enqueue the three tiers on the engine stream, bracketed by the engine's
 // events: ev_begin .. ev_mid is the primary tier, ev_mid .. ev_end the rescue.
-int enqueue_tiers(vd_plan* pl, int* launches, bool capturing = false) {
+// (Tiers::primary leaves the rescue out: the caller enqueues Tiers::rescue once it
+// has seen pairs on the primary tier's spill list.)
+enum class Tiers { all, primary, rescue };
+int enqueue_tiers(vd_plan* pl, int* launches, bool capturing = false, Tiers which = Tiers::all) {
   vd_engine* e = pl->eng;
   char* d = pl->base;
   const Layout& L = pl->L;
@@ -1092,8 +1127,10 @@ int enqueue_tiers(vd_plan* pl, int* launches, bool capturing = false) {
   // tier, cnt[9] head of the drift tier (FP32 semiglobal only), cnt[10]
   // head of the long-read kernel, cnt[11..12] its runs of strips and strips
   const int64_t long_tasks = pl->chunk.long_off.empty() ? 0 : pl->chunk.long_off.back();
-  VD_CUDA(cudaMemsetAsync(cnt, 0, L.o_lword - L.o_cnt + (size_t)long_tasks * sizeof(unsigned long long), pl->stream));
-  VD_CUDA(cudaEventRecordWithFlags(pl->ev_begin, pl->stream, evflags));
+  if (which != Tiers::rescue) {
+    VD_CUDA(cudaMemsetAsync(cnt, 0, L.o_lword - L.o_cnt + (size_t)long_tasks * sizeof(unsigned long long), pl->stream));
+    VD_CUDA(cudaEventRecordWithFlags(pl->ev_begin, pl->stream, evflags));
+  }
   const BatchView bv = batch_view(pl);
   // device tables by address; the scalars by value from the host copy
   TableSet* dt = (TableSet*)e->dtab.p;
@@ -1115,6 +1152,7 @@ int enqueue_tiers(vd_plan* pl, int* launches, bool capturing = false) {
   int n = 0;
   if (!pl->chunk.items.empty()) {
     cudaError_t err = cudaSuccess;
+    if (which != Tiers::rescue) {
     const int64_t np = pl->chunk.n_paired, nw = pl->chunk.n_paired_wide;
     const int64_t nl = pl->chunk.n_long;
     q.static_order = pl->params.schedule == VD_SCHEDULE_PLAIN ? 1 : 0;
@@ -1175,7 +1213,13 @@ int enqueue_tiers(vd_plan* pl, int* launches, bool capturing = false) {
     }
     if (nl > 0) VD_CUDA(cudaStreamWaitEvent(pl->stream, pl->side->join[0], 0));
     if (narrow_aside) VD_CUDA(cudaStreamWaitEvent(pl->stream, pl->side->join[1], 0));
+    }
     VD_CUDA(cudaEventRecordWithFlags(pl->ev_mid, pl->stream, evflags));
+    if (which == Tiers::primary) {
+      VD_CUDA(cudaEventRecordWithFlags(pl->ev_end, pl->stream, evflags));
+      if (launches) *launches = n;
+      return VD_OK;
+    }
     BatchView rv = bv;
     rv.hap_sel = nullptr;
     rv.out_sel = nullptr;
@@ -1406,18 +1450,8 @@ int vd_engine_create(int device, int64_t memory_mb, vd_engine** out) {
   if ((err = cudaStreamCreateWithPriority(&e->stream, cudaStreamNonBlocking, kOwnPriority)) != cudaSuccess ||
       (err = cudaEventCreate(&e->ev_begin)) != cudaSuccess || (err = cudaEventCreate(&e->ev_mid)) != cudaSuccess ||
       (err = cudaEventCreate(&e->ev_end)) != cudaSuccess ||
-      (err = e->side.create()) != cudaSuccess ||
       (err = cudaMallocHost((void**)&e->htab, sizeof(TableSet))) != cudaSuccess) {
     rc = cuda_fail(err, "engine setup");
-  }
-  for (int k = 0; k < 2 && !rc; ++k) {
-    vd_engine::Slot& sl = e->slots[k];
-    if ((err = cudaStreamCreateWithPriority(&sl.stream, cudaStreamNonBlocking, kOwnPriority)) != cudaSuccess ||
-        (err = cudaEventCreate(&sl.ev[0])) != cudaSuccess || (err = cudaEventCreate(&sl.ev[1])) != cudaSuccess ||
-        (err = cudaEventCreate(&sl.ev[2])) != cudaSuccess ||
-        (err = sl.side.create()) != cudaSuccess ||
-        (err = cudaMallocHost((void**)&sl.hcnt, 16 * sizeof(unsigned long long))) != cudaSuccess)
-      rc = cuda_fail(err, "engine pipeline setup");
   }
   if (!rc) rc = init_engine_grids(e);
   if (rc) { vd_engine_destroy(e); return rc; }
@@ -1521,6 +1555,10 @@ int vd_prefix_plan(const unsigned char* hap_bases, const int64_t* hap_off, int64
   return VD_OK;
 }
 
+// Batches up to this many cells (some tens of us of kernels) look before they launch
+// the rescue tiers.
+constexpr int64_t kDeferCells = 200'000'000;
+
 int vd_forward(vd_engine* e, const vd_batch* b, const vd_params* p, double* out, vd_stats* st) {
   const double t0 = now_ms();
   if (!e) return fail(VD_EINVAL, "engine is NULL");
@@ -1608,6 +1646,23 @@ int vd_forward(vd_engine* e, const vd_batch* b, const vd_params* p, double* out,
            64 * 1024;
   const int64_t budget = (int64_t)e->budget;
 
+  // a chunk's results and counters on their way back
+  auto fetch = [&](vd_engine::Slot& sl) -> int {
+    vd_plan& pl = *sl.pl;
+    const HostChunk& c = pl.chunk;
+    const double* dout = (const double*)(pl.base + pl.L.o_out);
+    if (c.n_out > 0) {
+      double* to = out + c.out_begin;
+      if (pair_form) {
+        sl.stage.resize((size_t)c.n_out);
+        to = sl.stage.data();
+      }
+      VD_CUDA(cudaMemcpyAsync(to, dout, (size_t)c.n_out * sizeof(double), cudaMemcpyDeviceToHost, sl.stream));
+      s.d2h_bytes += c.n_out * (int64_t)sizeof(double);
+    }
+    return enqueue_counter_read(&pl, sl.hcnt);
+  };
+
   // results of the chunk in a slot, once its stream has completed
   auto finish = [&](vd_engine::Slot& sl) -> int {
     if (!sl.busy) return VD_OK;
@@ -1615,7 +1670,30 @@ int vd_forward(vd_engine* e, const vd_batch* b, const vd_params* p, double* out,
     VD_CUDA(cudaStreamSynchronize(sl.stream));
     vd_plan& pl = *sl.pl;
     int64_t r0 = 0, r1 = 0, r2 = 0, lr = 0, ls = 0;
-    int r = check_counters(&pl, sl.hcnt, &r0, &r1, &r2, &lr, &ls);
+    int r;
+    if (sl.deferred && sl.hcnt[3] != 0 && sl.hcnt[5] == 0) {
+      double unused = 0.0;
+      if ((r = tier_times(&pl, &s.kernel_ms, &s.primary_ms, &unused))) return r;
+      int launches = 0;
+      if ((r = enqueue_tiers(&pl, &launches, false, Tiers::rescue))) return r;
+      s.kernel_launches += launches;
+      if ((r = fetch(sl))) return r;
+      VD_CUDA(cudaStreamSynchronize(sl.stream));
+      float ms = 0.f;
+      VD_CUDA(cudaEventElapsedTime(&ms, pl.ev_mid, pl.ev_end));
+      s.rescue_ms += ms;
+      s.kernel_ms += ms;
+      if ((r = check_counters(&pl, sl.hcnt, &r0, &r1, &r2, &lr, &ls))) return r;
+      s.long_strip_runs += lr;
+      s.long_strips += ls;
+      s.rescued_fp32 += r0;
+      s.rescued_fp64 += r1;
+      s.rescued_robust += r2;
+      const HostChunk& c = pl.chunk;
+      if (pair_form) for (int64_t k = 0; k < c.n_out; ++k) out[c.out_global[k]] = sl.stage[k];
+      return VD_OK;
+    }
+    r = check_counters(&pl, sl.hcnt, &r0, &r1, &r2, &lr, &ls);
     if (r) return r;
     if ((r = tier_times(&pl, &s.kernel_ms, &s.primary_ms, &s.rescue_ms))) return r;
     s.long_strip_runs += lr;
@@ -1648,6 +1726,7 @@ int vd_forward(vd_engine* e, const vd_batch* b, const vd_params* p, double* out,
     if (bytes > budget) return fail(VD_ENOMEM, "One pair exceeds CUDA workspace budget");
     vd_engine::Slot& sl = e->slots[chunk_index & 1];
     if ((rc = finish(sl))) return rc;  // the slot's previous chunk
+    VD_CUDA(sl.create());
     if (!sl.pl) sl.pl = new vd_plan();
     vd_plan& pl = *sl.pl;
     pl.chunk = HostChunk();
@@ -1670,23 +1749,18 @@ int vd_forward(vd_engine* e, const vd_batch* b, const vd_params* p, double* out,
     if ((rc = sl.arena.reserve(pl.L.total))) return rc;
     pl.base = (char*)sl.arena.p;
     s.live_bytes = std::max<int64_t>(s.live_bytes, (int64_t)(e->slots[0].arena.bytes + e->slots[1].arena.bytes));
-    if ((rc = upload_chunk(&pl, b, &s.h2d_bytes))) return rc;
+    if ((rc = upload_chunk(&pl, b, &s.h2d_bytes, sl.staging))) return rc;
     if (prev_end) VD_CUDA(cudaStreamWaitEvent(pl.stream, prev_end, 0));
+    // a small batch in one chunk launches its rescue tiers only when the counters
+    // that come back with the results show spilled pairs: three empty launches
+    // less where there are none, another round trip (some 20 us) where there are
+    const bool defer = chunk_index == 0 && u_end == units && c.cells < kDeferCells;
     int launches = 0;
-    if ((rc = enqueue_tiers(&pl, &launches))) return rc;
+    if ((rc = enqueue_tiers(&pl, &launches, false, defer ? Tiers::primary : Tiers::all))) return rc;
     prev_end = pl.ev_end;
-    s.kernel_launches += launches + (c.n_out > 0 ? 1 : 0);  // the -inf fill of the upload
-    const double* dout = (const double*)(pl.base + pl.L.o_out);
-    if (c.n_out > 0) {
-      if (pair_form) {
-        sl.stage.resize((size_t)c.n_out);
-        VD_CUDA(cudaMemcpyAsync(sl.stage.data(), dout, (size_t)c.n_out * sizeof(double), cudaMemcpyDeviceToHost, sl.stream));
-      } else {
-        VD_CUDA(cudaMemcpyAsync(out + c.out_begin, dout, (size_t)c.n_out * sizeof(double), cudaMemcpyDeviceToHost, sl.stream));
-      }
-      s.d2h_bytes += c.n_out * (int64_t)sizeof(double);
-    }
-    if ((rc = enqueue_counter_read(&pl, sl.hcnt))) return rc;
+    sl.deferred = defer;
+    s.kernel_launches += launches + (pl.filled ? 1 : 0);  // the -inf fill of the upload
+    if ((rc = fetch(sl))) return rc;
     sl.busy = true;
     s.dp_cells += c.cells;
     s.shared_cells += c.shared_cells;
@@ -1710,6 +1784,7 @@ namespace {
 int enqueue_whole(vd_engine* e, const vd_batch* b, const vd_params* p, vd_engine::Slot& sl, vd_stats* s) {
   int rc = ensure_tables(e, p);
   if (rc) return rc;
+  VD_CUDA(sl.create());
   if (!sl.pl) sl.pl = new vd_plan();
   vd_plan& pl = *sl.pl;
   pl.chunk = HostChunk();
@@ -1730,7 +1805,7 @@ int enqueue_whole(vd_engine* e, const vd_batch* b, const vd_params* p, vd_engine
   s->host_ms += now_ms() - th;
   if ((rc = sl.arena.reserve(pl.L.total))) return rc;
   pl.base = (char*)sl.arena.p;
-  if ((rc = upload_chunk(&pl, b, &s->h2d_bytes))) return rc;
+  if ((rc = upload_chunk(&pl, b, &s->h2d_bytes, sl.staging))) return rc;
   int launches = 0;
   if ((rc = enqueue_tiers(&pl, &launches))) return rc;
   if ((rc = enqueue_counter_read(&pl, sl.hcnt))) return rc;
@@ -1754,6 +1829,7 @@ int vd_plan_create(vd_engine* e, const vd_batch* b, const vd_params* p, vd_plan*
   std::lock_guard<std::mutex> lk(e->mu);
   DeviceGuard guard(e->device);
   if ((rc = ensure_tables(e, p))) return rc;
+  VD_CUDA(e->side.create());
   vd_plan* pl = new vd_plan();
   pl->eng = e;
   pl->params = *p;
@@ -2023,6 +2099,7 @@ int vd_forward_backward(vd_engine* e, const vd_batch* b, const vd_params* p, int
     gv.count = nullptr;
     const bool aside = n_kernel[0] && n_kernel[1];
     if (aside) {
+      VD_CUDA(e->side.create());
       VD_CUDA(cudaEventRecord(e->side.fork, st_));
       VD_CUDA(cudaStreamWaitEvent(e->side.s[1], e->side.fork, 0));
     }
@@ -2149,7 +2226,7 @@ int vd_region_genotypes(vd_engine* e, const vd_batch* b, const vd_params* p, con
       vd_engine* e;
       vd_engine::Slot& sl;
       ~Drain() {
-        cudaStreamSynchronize(sl.stream);
+        if (sl.stream) cudaStreamSynchronize(sl.stream);
         if (sl.arena.bytes > e->budget) sl.arena.release();  // (this call ignores the memory budget)
       }
     } drain{e, sl};
