@@ -21,12 +21,14 @@
 //  4. scores the region batch with vd_forward and scatters the results back
 //     to the input order.
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
 #include <memory>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/vardepth_pairhmm.h"
@@ -34,6 +36,18 @@
 
 namespace vd {
 namespace {
+
+// fn(begin, end) over [0, n) on up to 8 host threads, in slices of at least `grain`
+// (the calling thread takes the first); a thread costs some 20 us to start.
+template <typename F>
+void in_slices(int64_t n, int64_t grain, F&& fn) {
+  const int64_t hw = std::max<int64_t>(1, (int64_t)std::thread::hardware_concurrency());
+  const int64_t T = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(hw, 8), n / grain));
+  std::vector<std::thread> th;
+  for (int64_t k = 1; k < T; ++k) th.emplace_back([&fn, n, k, T] { fn(n * k / T, n * (k + 1) / T); });
+  fn((int64_t)0, n / T);
+  for (auto& x : th) x.join();
+}
 
 // every byte one of A, C, G, T, N (comparisons the compiler vectorises)
 bool is_dna(const unsigned char* p, int n) {
@@ -106,76 +120,81 @@ class IdTable {
 };
 
 // Distinct byte strings (a read is its bases and qualities, a haplotype its
-// bases): ids in order of first appearance.  A direct-mapped cache of recent
-// pointers answers repeats of the same object (a caller passes each read's
-// objects with every haplotype, and the same few haplotype objects over and
-// over); a new pointer is checked for ACGTN and looked up by content.
+// bases): ids in order of first appearance.  note() gives every object seen an
+// index, answering repeats of the same pointer from a direct-mapped cache of recent
+// ones (a caller passes each read's objects with every haplotype, and the same few
+// haplotype objects over and over); resolve() then checks the new objects for ACGTN
+// and hashes them, on several threads, and looks them up by content in order.
 class Interner {
  public:
   std::vector<const unsigned char*> bases, quals;
   std::vector<int> len;
 
   // track_pointers: keep every pointer seen (haplotype objects recur all over
-  // a pair list); without it a pointer evicted from the cache is looked up by
-  // content again (a read's object recurs only in its own run of pairs)
+  // a pair list); without it a pointer evicted from the cache counts as a new
+  // object (a read's object recurs only in its own run of pairs)
   explicit Interner(bool track_pointers) : track_(track_pointers) {}
 
-  // id of (b, q, n); -1 when the bases are not uppercase ACGTN
-  int32_t id(const unsigned char* b, const unsigned char* q, int n) {
+  // index of the object (b, q, n)
+  int32_t note(const unsigned char* b, const unsigned char* q, int n) {
     uint64_t hp = ((uint64_t)(uintptr_t)b * 0x9e3779b97f4a7c15ull) ^ ((uint64_t)(uintptr_t)q * 0xc2b2ae3d27d4eb4full) ^
                   (uint64_t)n;
     hp ^= hp >> 29;
-    Slot& c = cache_[hp & (kCache - 1)];
-    if (c.id >= 0 && c.b == b && c.q == q && c.n == n) return c.id;
+    int32_t& c = cache_[hp & (kCache - 1)];
+    auto same = [&](int32_t k) {
+      const Object& x = objects_[(size_t)k];
+      return x.b == b && x.q == q && x.n == n;
+    };
+    if (c >= 0 && same(c)) return c;
     if (track_) {  // a pointer seen before, evicted from the cache
-      const int32_t e = by_ptr_.find(hp, [&](int32_t k) {
-        const Slot& x = ptrs_[(size_t)k];
-        return x.b == b && x.q == q && x.n == n;
-      });
-      if (e >= 0) {
-        c = ptrs_[(size_t)e];
-        return c.id;
-      }
+      const int32_t e = by_ptr_.find(hp, same);
+      if (e >= 0) return c = e;
     }
-    const int32_t r = by_content(b, q, n);
-    if (r < 0) return -1;
-    c = Slot{b, q, n, r};
-    if (track_) {
-      by_ptr_.insert(hp, (int32_t)ptrs_.size());
-      ptrs_.push_back(c);
-    }
-    return r;
+    c = (int32_t)objects_.size();
+    objects_.push_back(Object{b, q, n, -1, 0});
+    if (track_) by_ptr_.insert(hp, c);
+    return c;
   }
+
+  // ids of all objects noted; id() is -1 where the bases are not uppercase ACGTN
+  void resolve() {
+    in_slices((int64_t)objects_.size(), 2048, [&](int64_t lo, int64_t hi) {
+      for (int64_t k = lo; k < hi; ++k) {
+        Object& x = objects_[(size_t)k];
+        x.id = is_dna(x.b, x.n) ? 0 : -1;
+        x.h = x.n ? hash_bytes(x.b, x.n, 0x51ed27e5u) : 0x51ed27e5u;
+        if (x.q && x.n) x.h = hash_bytes(x.q, x.n, x.h);
+      }
+    });
+    for (Object& x : objects_) {
+      if (x.id < 0) continue;
+      x.id = by_content_.find(x.h, [&](int32_t j) {
+        return len[(size_t)j] == x.n &&
+               (x.n == 0 || (std::memcmp(bases[(size_t)j], x.b, (size_t)x.n) == 0 &&
+                             (!x.q || std::memcmp(quals[(size_t)j], x.q, (size_t)x.n) == 0)));
+      });
+      if (x.id >= 0) continue;
+      x.id = (int32_t)len.size();
+      bases.push_back(x.b);
+      quals.push_back(x.q);
+      len.push_back(x.n);
+      by_content_.insert(x.h, x.id);
+    }
+  }
+  int32_t id(int32_t object) const { return objects_[(size_t)object].id; }
 
  private:
-  int32_t by_content(const unsigned char* b, const unsigned char* q, int n) {
-    if (!is_dna(b, n)) return -1;
-    uint64_t h = n ? hash_bytes(b, n, 0x51ed27e5u) : 0x51ed27e5u;
-    if (q && n) h = hash_bytes(q, n, h);
-    int32_t r = by_content_.find(h, [&](int32_t j) {
-      return len[(size_t)j] == n && (n == 0 || (std::memcmp(bases[(size_t)j], b, (size_t)n) == 0 &&
-                                                (!q || std::memcmp(quals[(size_t)j], q, (size_t)n) == 0)));
-    });
-    if (r < 0) {
-      r = (int32_t)len.size();
-      bases.push_back(b);
-      quals.push_back(q);
-      len.push_back(n);
-      by_content_.insert(h, r);
-    }
-    return r;
-  }
-
-  struct Slot {
-    const unsigned char* b = nullptr;
-    const unsigned char* q = nullptr;
-    int n = -1;
-    int32_t id = -1;
+  struct Object {
+    const unsigned char* b;
+    const unsigned char* q;
+    int n;
+    int32_t id;
+    uint64_t h;
   };
   static constexpr size_t kCache = 4096;
-  std::vector<Slot> cache_ = std::vector<Slot>(kCache);
+  std::vector<int32_t> cache_ = std::vector<int32_t>(kCache, -1);
   bool track_;
-  std::vector<Slot> ptrs_;  // every distinct (pointer, length) seen, with its id
+  std::vector<Object> objects_;
   IdTable by_ptr_, by_content_;
 };
 
@@ -196,17 +215,39 @@ int build_plan(const char* const* rs, const unsigned char* const* qs, const int*
                const int* hn, int64_t count, PairListPlan& pl) {
   pl.pair_read.resize((size_t)count);
   pl.pair_hap.resize((size_t)count);
-  for (int64_t p = 0; p < count; ++p) {
+  // (the objects of the pairs before the first malformed one: an earlier pair that
+  // is not DNA is reported before it)
+  int64_t good = 0;
+  std::string malformed;
+  for (; good < count; ++good) {
+    const int64_t p = good;
     const int n = rn[p], m = hn[p];
-    if (n < 0 || m < 0) return report_error(VD_EINVAL, ("negative length at pair " + std::to_string(p)).c_str());
-    if ((n > 0 && (!rs[p] || !qs[p])) || (m > 0 && !hs[p]))
-      return report_error(VD_EINVAL, ("NULL sequence at pair " + std::to_string(p)).c_str());
-    const int32_t r = pl.reads.id((const unsigned char*)rs[p], qs[p], n);
-    const int32_t h = pl.haps.id((const unsigned char*)hs[p], nullptr, m);
-    if (r < 0 || h < 0) return report_error(VD_EINVAL, "Uppercase DNA required");
-    pl.pair_read[(size_t)p] = r;
-    pl.pair_hap[(size_t)p] = h;
+    if (n < 0 || m < 0) {
+      malformed = "negative length at pair " + std::to_string(p);
+      break;
+    }
+    if ((n > 0 && (!rs[p] || !qs[p])) || (m > 0 && !hs[p])) {
+      malformed = "NULL sequence at pair " + std::to_string(p);
+      break;
+    }
+    pl.pair_read[(size_t)p] = pl.reads.note((const unsigned char*)rs[p], qs[p], n);
+    pl.pair_hap[(size_t)p] = pl.haps.note((const unsigned char*)hs[p], nullptr, m);
   }
+  pl.reads.resolve();
+  pl.haps.resolve();
+  std::atomic<bool> dna{true};
+  in_slices(good, 32768, [&](int64_t lo, int64_t hi) {
+    bool ok = true;
+    for (int64_t p = lo; p < hi; ++p) {
+      const int32_t r = pl.reads.id(pl.pair_read[(size_t)p]), h = pl.haps.id(pl.pair_hap[(size_t)p]);
+      pl.pair_read[(size_t)p] = r;
+      pl.pair_hap[(size_t)p] = h;
+      ok &= r >= 0 && h >= 0;
+    }
+    if (!ok) dna = false;
+  });
+  if (!dna) return report_error(VD_EINVAL, "Uppercase DNA required");
+  if (good < count) return report_error(VD_EINVAL, malformed.c_str());
   // each read's distinct haplotypes (counting sort by read, then sort + unique)
   const int64_t nr = (int64_t)pl.reads.len.size();
   std::vector<int64_t> start((size_t)nr + 1, 0);
@@ -274,7 +315,8 @@ int build_plan(const char* const* rs, const unsigned char* const* qs, const int*
   // output slot of every input pair
   pl.pair_region.resize((size_t)count);
   pl.pair_slot.resize((size_t)count);
-  for (int64_t p = 0; p < count; ++p) {
+  in_slices(count, 16384, [&](int64_t lo, int64_t hi) {
+   for (int64_t p = lo; p < hi; ++p) {
     const int32_t r = pl.pair_read[(size_t)p];
     const int32_t g = pl.read_region[(size_t)r];
     const int32_t* hb = pl.region_haps.data() + pl.region_hap_off[(size_t)g];
@@ -282,7 +324,8 @@ int build_plan(const char* const* rs, const unsigned char* const* qs, const int*
     const int64_t j = std::lower_bound(hb, hb + nh, pl.pair_hap[(size_t)p]) - hb;
     pl.pair_region[(size_t)p] = g;
     pl.pair_slot[(size_t)p] = pl.region_out_off[(size_t)g] + (int64_t)local[(size_t)r] * nh + j;
-  }
+   }
+  });
   return VD_OK;
 }
 
