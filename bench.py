@@ -250,6 +250,13 @@ def reference_arm(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
         return
+    from oracle import oracle as O
+    if not O.ref_available():
+        O.build()
+    if not O.ref_available():
+        print(json.dumps({"impl": "reference", "unavailable": "the reference's libraries (oracle/_ref) are not built "
+                          "and its sources are not here"}), flush=True)
+        return
     w = make_workload(args.workload, args.regions)
     per_step = max(2.0, args.cpu_seconds)
     res = cpu_reference(w, per_step, repeats=0)
@@ -697,9 +704,13 @@ def main():
     if rank == 0 and world == 1:
         res = None
         if not args.no_cpu:
-            res = cpu_reference(w, args.cpu_seconds)
-            cpu = {"value": round(res["cells"] / res["times"][0] / 1e9, 4), "unit": "GCUPS", "cores": res["threads"],
-                   "kind": "reference", "sample": res["sample"]}
+            try:
+                res = cpu_reference(w, args.cpu_seconds)
+            except FileNotFoundError as e:  # the reference's libraries were not built here
+                cpu = {"unavailable": str(e)}
+            else:
+                cpu = {"value": round(res["cells"] / res["times"][0] / 1e9, 4), "unit": "GCUPS",
+                       "cores": res["threads"], "kind": "reference", "sample": res["sample"]}
         parity = {}
         region_cells = shard.region_cells(full)
         if res is not None:
