@@ -9,7 +9,7 @@
 //
 // Work decomposition.  A warp owns one read (n rows) and streams through a list
 // of K haplotypes.  Lane L owns R consecutive rows of the current strip of
-// 32*R rows (reads longer than 256 bases are strip-mined with R = 8); the
+// 32*R rows (longer reads are strip-mined); the
 // placement of the read in the strip is described at process_item.  At step
 // t lane L is at position p = t - L of the "column stream": haplotype k
 // occupies positions S_k (its column 0) .. S_k + m_k.  Consecutive haplotypes
@@ -68,7 +68,7 @@ inline __host__ __device__ int make_code(int R, bool general, bool multistrip) {
   return R | (general ? 256 : 0) | (multistrip ? 512 : 0);
 }
 constexpr int kPairedBit = 1024;
-constexpr int kLongBit = 2048;  // a long read against one or two haplotypes (pairhmm_long.cuh)
+constexpr int kLongBit = 2048;  // a long read against up to kLongGroupMax haplotypes (pairhmm_long.cuh)
 inline __host__ __device__ bool code_long(int c) { return (c >> 11) & 1; }
 
 // Per-quality tables (index = raw Phred byte) and scalar constants for one
@@ -125,7 +125,7 @@ struct QueueView {
   long long scratch_stride;   // in boundary records (float2 / double2)
   int* error_flag;            // set when the spill list overflows
   int static_order;           // 1: warp w takes items w, w + W, w + 2W ... (W = warps in the grid)
-  unsigned long long* strip_runs;  // long-read kernel, nullable: [0] runs of strips, [1] strips
+  unsigned long long* strip_runs;  // long-read kernel, nullable: [0] runs of strips, [1] strips (equal)
   // long-read kernel: tasks (strips of pairs), the number of each item's first
   // task, one word per task (pairhmm_long.cuh), and where a boundary buffer's
   // block exponents start (in 16-byte records)

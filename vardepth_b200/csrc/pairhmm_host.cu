@@ -231,8 +231,6 @@ struct vd_engine {
   bool tvalid = false;
   TableSet* htab = nullptr;   // pinned host copy
   DevBuf dtab;
-  // batch arena reused by vd_forward
-  DevBuf arena;
   std::vector<double> out_stage;
   // live plans: destroying the engine first releases their device resources
   std::unordered_set<vd_plan*> plans;
@@ -704,7 +702,7 @@ void build_region_chunk(const vd_batch* b, int64_t g0, int64_t g1, const TableSe
                               c.hap_share.data() + (h_lo - c.ha));
     // a long read (FP32 semiglobal, one-sided emission) against its region's
     // non-empty haplotypes: runs of up to long_group neighbours per item, in
-    // both schedules (two of an item share a warp)
+    // both schedules (two of an item share a warp, a strip of the two is a task)
     auto emit_long = [&](int64_t r) {
       const int32_t code = c.read_code[r - c.ra];
       const int n = (int)(c.read_off[r - c.ra + 1] - c.read_off[r - c.ra]);
@@ -1485,7 +1483,6 @@ int vd_engine_destroy(vd_engine* e) {
       sl.side.destroy();
       if (sl.stream) cudaStreamDestroy(sl.stream);
     }
-    e->arena.release();
     e->grad_arena.release();
     e->geno_arena.release();
     e->dtab.release();

@@ -52,8 +52,11 @@ constexpr size_t na_align(size_t v) { return (v + 255) / 256 * 256; }
 
 // Layout of the static scratch (byte offsets).
 constexpr size_t kOffCnt = 0;  // 16 x u64: [0..2] work heads, [3],[4] spill counts, [5] overflow,
-                               // [8] length error, [9] non-empty haplotypes
-constexpr size_t kOffTab32 = 256;
+                               // [8] length error, [9] non-empty haplotypes,
+                               // [16 + k] reads of class k, [25 + k] those placed (na_units)
+constexpr int kNaCounters = 16 + 9 + 9;
+constexpr size_t kOffTab32 = 512;
+static_assert(kNaCounters * 8 <= kOffTab32, "the counters end before the tables");
 constexpr size_t kOffTab64 = na_align(kOffTab32 + sizeof(Tables<float>));
 constexpr size_t kOffCode = na_align(kOffTab64 + sizeof(Tables<double>));
 constexpr size_t kOffHapSel = na_align(kOffCode + sizeof(int32_t) * kNaMaxReads);
@@ -61,6 +64,10 @@ constexpr size_t kOffOutSel = na_align(kOffHapSel + sizeof(int32_t) * kNaMaxHaps
 constexpr size_t kOffSpill1 = na_align(kOffOutSel + sizeof(int64_t) * kNaMaxPairs);
 constexpr size_t kOffSpill2 = na_align(kOffSpill1 + sizeof(RescueEntry) * kNaMaxPairs);
 constexpr size_t kOffStrip = na_align(kOffSpill2 + sizeof(RescueEntry) * kNaMaxPairs);
+// The two-read tier's units lie where the robust tier, which starts after it, keeps
+// its strips.
+constexpr size_t kOffUnits = kOffStrip;
+static_assert(sizeof(int2) * kNaMaxReads <= sizeof(double2) * (kNaMaxHapLen + 1) * kNaRobustWarps, "units fit");
 constexpr size_t kNoAllocBytes = na_align(kOffStrip + sizeof(double2) * (kNaMaxHapLen + 1) * kNaRobustWarps);
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
@@ -112,10 +119,11 @@ __global__ void na_prep_haps(const int64_t* __restrict__ hap_off, int n_haps, un
   if (threadIdx.x == 0) cnt[9] = (unsigned long long)base;
 }
 
-// Per-read kernel codes, length checks, -inf for every output, and the output
-// slot of every (read, non-empty haplotype).
+// Per-read kernel codes (a warp per read: its qualities are looked up side by
+// side), length checks, -inf for every output, and the output slot of every
+// (read, non-empty haplotype).
 __global__ void na_prep_reads(const unsigned char* __restrict__ read_quals, const int64_t* __restrict__ read_off,
-                              int n_reads, int n_haps, int anchored, double* __restrict__ out,
+                              int n_reads, int n_haps, int anchored, int classes, double* __restrict__ out,
                               unsigned char* scratch) {
   unsigned long long* cnt = reinterpret_cast<unsigned long long*>(scratch + kOffCnt);
   const Tables<float>* tab = reinterpret_cast<const Tables<float>*>(scratch + kOffTab32);
@@ -125,15 +133,24 @@ __global__ void na_prep_reads(const unsigned char* __restrict__ read_quals, cons
   const int nh_ne = (int)cnt[9];
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  for (int64_t r = tid; r < n_reads; r += stride) {
+  const int lane = threadIdx.x & (kWarp - 1);
+  for (int64_t r = tid / kWarp; r < n_reads; r += stride / kWarp) {
     const int64_t o = read_off[r];
     const int64_t n = read_off[r + 1] - o;
-    if (n > kNaMaxReadLen || n < 0) atomicCAS(&cnt[8], 0ull, 1ull);
     bool gen = false;
-    for (int64_t i = 0; i < n && i < kNaMaxReadLen; ++i) gen |= tab->general[read_quals[o + i]] != 0;
-    const int rows = (int)n + anchored;
-    const int R = min(kMaxR, max(1, (rows + kWarp - 1) / kWarp));
-    code[r] = make_code(R, gen, false);
+#pragma unroll
+    for (int i = 0; i < kNaMaxReadLen; i += kWarp) {
+      const int64_t k = i + lane;
+      if (k < n && k < kNaMaxReadLen) gen |= tab->general[read_quals[o + k]] != 0;
+    }
+    gen = __any_sync(0xffffffffu, gen);
+    if (lane == 0) {
+      if (n > kNaMaxReadLen || n < 0) atomicCAS(&cnt[8], 0ull, 1ull);
+      const int rows = (int)n + anchored;
+      const int R = min(kMaxR, max(1, (rows + kWarp - 1) / kWarp));
+      code[r] = make_code(R, gen, false);
+      if (classes && n > 0) atomicAdd(&cnt[16 + (gen ? 8 : R - 1)], 1ull);
+    }
   }
   for (int64_t k = tid; k < (int64_t)n_reads * n_haps; k += stride) out[k] = -HUGE_VAL;
   for (int64_t k = tid; k < (int64_t)n_reads * nh_ne; k += stride) {
@@ -142,12 +159,39 @@ __global__ void na_prep_reads(const unsigned char* __restrict__ read_quals, cons
   }
 }
 
+// Units of the two-read tier: reads of one class (rows per lane, one-sided
+// emission) by twos, the odd one and the reads with two-sided emission (class 8)
+// alone, with -1 in the partner's place.  A class's units follow those of the class
+// with more rows.  Which reads meet changes no bit of a result.
+__device__ __forceinline__ int na_class_units(const unsigned long long* cnt, int k) {
+  return k == 8 ? (int)cnt[16 + k] : ((int)cnt[16 + k] + 1) / 2;
+}
+__global__ void na_units(const int64_t* __restrict__ read_off, int n_reads, unsigned char* scratch) {
+  unsigned long long* cnt = reinterpret_cast<unsigned long long*>(scratch + kOffCnt);
+  const int32_t* code = reinterpret_cast<const int32_t*>(scratch + kOffCode);
+  int* units = reinterpret_cast<int*>(scratch + kOffUnits);
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (cnt[8] != 0 || r >= n_reads || read_off[r + 1] == read_off[r]) return;
+  const int k = code_general(code[r]) ? 8 : code_R(code[r]) - 1;
+  int base = 0;
+  for (int c = 8; c > k; --c) base += na_class_units(cnt, c);
+  const int at = (int)atomicAdd(&cnt[25 + k], 1ull);
+  const int of = (int)cnt[16 + k];
+  if (k == 8) {
+    units[2 * (base + at)] = r;
+    units[2 * (base + at) + 1] = -1;
+  } else {
+    units[2 * base + at] = r;
+    if (at == of - 1 && (of & 1)) units[2 * base + of] = -1;
+  }
+}
+
 // Primary tier over the region: work item i is read i / pieces against its share
 // of the non-empty haplotypes (the (i mod pieces)-th of `pieces` runs), derived
 // here instead of read from a host-built list.  Reads alone leave most of the
 // GPU idle (301 reads x 13 haplotypes of 421 bases: 1.10 ms with one item per
-// read, a serial chain of 5,500 columns); the call asks for about four items
-// per resident warp.
+// read, a serial chain of 5,500 columns; 0.36 by pieces); the call asks for about
+// four items per resident warp.  FP64 and anchored mode (na_pairs: the rest).
 template <typename T, bool ANCH>
 __global__ void __launch_bounds__(kWarpsPerBlock * kWarp, MinBlocks<T>::value)
 na_primary(const __grid_constant__ BatchView bv, const __grid_constant__ QueueView qv,
@@ -190,6 +234,79 @@ na_primary(const __grid_constant__ BatchView bv, const __grid_constant__ QueueVi
   }
 }
 
+// The same in FP32 semiglobal mode: work item i is unit i / pieces against its share
+// of the haplotypes.  With `paired` the units are those of na_units, two reads per
+// warp in packed FP32 where their class has two; without, unit u is read u.  Issue
+// slots bound the single-read kernel here (at 96 registers its rows spill); two
+// reads per warp halve them: 301 reads x 13 haplotypes of 421 bases 360 -> 260 us a
+// call, 700 x 24 of 1,000 1,866 -> 990.  A call with fewer (read, haplotype) pairs than
+// eight per SM leaves each scheduler a warp or two, whose steps alone are shorter
+// with one read (30 x 24 of 1,000: 282 us alone, 305 by twos; 100 x 16 of 300: 241 and
+// 217).  About eight items per resident warp are asked for: fewer leave a longer tail
+// (700 x 24: 1,228, 1,158, 1,093, 990 us at 1, 2, 4, 8), more are no faster.
+__global__ void __launch_bounds__(kWarpsPerBlock * kWarp, 3)
+na_pairs(const __grid_constant__ BatchView bv, const __grid_constant__ QueueView qv,
+         const __grid_constant__ Scalars<float> sc, int n_reads, int n_haps, int pieces, int paired,
+         unsigned char* scratch) {
+  __shared__ Tables<float> tab;
+  __shared__ float4 saves[kWarpsPerBlock][(kMaxR + 2) * kWarp];
+  __shared__ HapMeta meta[kWarpsPerBlock][kMetaRing];
+  {
+    const int words = (int)(sizeof(Tables<float>) / sizeof(int));
+    const int* src = reinterpret_cast<const int*>(scratch + kOffTab32);
+    int* dst = reinterpret_cast<int*>(&tab);
+    for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
+  }
+  __syncthreads();
+  const unsigned long long* cnt = reinterpret_cast<const unsigned long long*>(scratch + kOffCnt);
+  if (cnt[8] != 0) return;  // a length limit was exceeded: nothing runs
+  const int2* units = reinterpret_cast<const int2*>(scratch + kOffUnits);
+  const int nh_ne = (int)cnt[9];
+  int n_units = n_reads;
+  if (paired) {
+    n_units = 0;
+    for (int k = 0; k < 9; ++k) n_units += na_class_units(cnt, k);
+  }
+  const int lane = threadIdx.x & (kWarp - 1), wid = threadIdx.x >> 5;
+  BatchView pv = bv;  // the two-read items take haplotype k, and its output column, from the list
+  pv.hap_order = bv.hap_sel;
+  for (;;) {
+    unsigned long long i = 0;
+    if (lane == 0) i = atomicAdd(qv.head, 1ull);
+    i = __shfl_sync(0xffffffffu, i, 0);
+    if ((long long)i >= (long long)n_units * pieces) break;
+    const int u = (int)(i / pieces), piece = (int)(i % pieces);
+    const int h0 = (int)((long long)nh_ne * piece / pieces), h1 = (int)((long long)nh_ne * (piece + 1) / pieces);
+    if (h1 <= h0) continue;
+    const int2 rr = paired ? units[u] : make_int2(u, -1);
+    if (bv.read_off[rr.x + 1] <= bv.read_off[rr.x]) continue;
+    ItemRef it;
+    it.w.read = rr.x;
+    it.w.nhap = h1 - h0;
+    it.w.hap_begin = h0;
+    it.w.code = bv.read_code[rr.x];
+    it.w.read2 = rr.y;
+    it.tier = 0;
+    if (rr.y < 0) {
+      it.w.out_begin = (int64_t)rr.x * nh_ne + h0;
+      it.w.out2_begin = 0;
+      it.use_sel = true;
+      dispatch<float, false>(it.w.code, bv, qv, it, &tab, sc, lane, reinterpret_cast<float2*>(qv.scratch));
+      continue;
+    }
+    it.w.out_begin = (int64_t)rr.x * n_haps;
+    it.w.out2_begin = (int64_t)rr.y * n_haps;
+    it.use_sel = false;
+    switch (code_R(it.w.code)) {
+#define VD_PCASE(r) \
+      case r: process_pair<r>(pv, qv, it, &tab, sc, lane, saves[wid], meta[wid]); break;
+      VD_PCASE(1) VD_PCASE(2) VD_PCASE(3) VD_PCASE(4) VD_PCASE(5) VD_PCASE(6) VD_PCASE(7) VD_PCASE(8)
+#undef VD_PCASE
+      default: break;
+    }
+  }
+}
+
 }  // namespace
 }  // namespace vd
 
@@ -206,8 +323,10 @@ struct NaDevice {
   bool tables = false;               // ... that the scratch on the device holds
   bool ready = false;
   unsigned char* scratch = nullptr;  // device address of g_noalloc_scratch on this device
-  int grid32[2] = {0, 0};            // [anchored] blocks of na_primary<float>
+  int grid32 = 0;                    // blocks of na_primary<float>
   int grid64[2] = {0, 0};            // [anchored] blocks of na_primary<double>
+  int grid_pairs = 0;                // blocks of na_pairs
+  int sms = 0;
   int rescue[2] = {0, 0};            // [anchored] blocks of the FP64 rescue tier
 };
 constexpr int kNaMaxDevices = 64;
@@ -248,14 +367,15 @@ int na_setup(int device) {
   d.scratch = static_cast<unsigned char*>(ptr);
   int sms = 0, b = 0;
   NA_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-  NA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, na_primary<float, false>, kWarpsPerBlock * kWarp, 0));
-  d.grid32[0] = std::max(1, b) * sms;
   NA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, na_primary<float, true>, kWarpsPerBlock * kWarp, 0));
-  d.grid32[1] = std::max(1, b) * sms;
+  d.grid32 = std::max(1, b) * sms;
   NA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, na_primary<double, false>, kWarpsPerBlock * kWarp, 0));
   d.grid64[0] = std::max(1, b) * sms;
   NA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, na_primary<double, true>, kWarpsPerBlock * kWarp, 0));
   d.grid64[1] = std::max(1, b) * sms;
+  NA_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, na_pairs, kWarpsPerBlock * kWarp, 0));
+  d.grid_pairs = std::max(1, b) * sms;
+  d.sms = sms;
   for (int a = 0; a < 2; ++a) {
     NA_CUDA(occupancy_f64(a != 0, &b));
     d.rescue[a] = std::max(1, b) * sms;
@@ -346,14 +466,21 @@ extern "C" int vd_forward_region_noalloc(int device, const unsigned char* read_b
   }
   const Scalars<float>& s32 = d.s32;
   const Scalars<double>& s64 = d.s64;
+  // semiglobal FP32: two reads per warp (na_pairs) once eight pairs per SM are asked for
+  const bool packed = !f64 && !anch;
+  const bool paired = packed && n_reads * n_haps >= 8 * (int64_t)d.sms;
   // the previous call's counters and lists are still in the array: the
   // counters are cleared here; the lists are only read up to their counts
-  NA_CUDA(cudaMemsetAsync(sc + kOffCnt, 0, 16 * sizeof(unsigned long long), s));
+  NA_CUDA(cudaMemsetAsync(sc + kOffCnt, 0, kNaCounters * sizeof(unsigned long long), s));
   na_prep_haps<<<1, 256, 0, s>>>(hap_off, (int)n_haps, sc);
   NA_CUDA(cudaGetLastError());
-  na_prep_reads<<<(int)std::min<int64_t>(1024, (n_reads * n_haps + 255) / 256 + 1), 256, 0, s>>>(
-      read_quals, read_off, (int)n_reads, (int)n_haps, anch ? 1 : 0, out, sc);
+  na_prep_reads<<<(int)std::min<int64_t>(1024, std::max((n_reads * n_haps + 255) / 256, (n_reads + 7) / 8)), 256, 0, s>>>(
+      read_quals, read_off, (int)n_reads, (int)n_haps, anch ? 1 : 0, paired ? 1 : 0, out, sc);
   NA_CUDA(cudaGetLastError());
+  if (paired) {
+    na_units<<<(int)((n_reads + 255) / 256), 256, 0, s>>>(read_off, (int)n_reads, sc);
+    NA_CUDA(cudaGetLastError());
+  }
 
   unsigned long long* cnt = reinterpret_cast<unsigned long long*>(sc + kOffCnt);
   BatchView bv{};
@@ -376,14 +503,17 @@ extern "C" int vd_forward_region_noalloc(int device, const unsigned char* read_b
   q.scratch_stride = kNaMaxHapLen + 1;
   q.error_flag = reinterpret_cast<int*>(cnt + 5);
   // primary tier: FP32 (or FP64 when asked), work items derived on the device
-  const int64_t warps = (int64_t)(f64 ? d.grid64 : d.grid32)[anch] * kWarpsPerBlock;
-  const int pieces = (int)std::max<int64_t>(1, std::min<int64_t>(n_haps, 4 * warps / n_reads));
-  if (f64) {
+  const int64_t warps = (int64_t)(packed ? d.grid_pairs : f64 ? d.grid64[anch] : d.grid32) * kWarpsPerBlock;
+  const int64_t units = paired ? (n_reads + 1) / 2 : n_reads;
+  const int pieces = (int)std::max<int64_t>(1, std::min<int64_t>(n_haps, (packed ? 8 : 4) * warps / units));
+  if (packed) {
+    na_pairs<<<d.grid_pairs, kWarpsPerBlock * kWarp, 0, s>>>(bv, q, s32, (int)n_reads, (int)n_haps, pieces,
+                                                             paired ? 1 : 0, sc);
+  } else if (f64) {
     if (anch) na_primary<double, true><<<d.grid64[1], kWarpsPerBlock * kWarp, 0, s>>>(bv, q, s64, (int)n_reads, pieces, sc);
     else na_primary<double, false><<<d.grid64[0], kWarpsPerBlock * kWarp, 0, s>>>(bv, q, s64, (int)n_reads, pieces, sc);
   } else {
-    if (anch) na_primary<float, true><<<d.grid32[1], kWarpsPerBlock * kWarp, 0, s>>>(bv, q, s32, (int)n_reads, pieces, sc);
-    else na_primary<float, false><<<d.grid32[0], kWarpsPerBlock * kWarp, 0, s>>>(bv, q, s32, (int)n_reads, pieces, sc);
+    na_primary<float, true><<<d.grid32, kWarpsPerBlock * kWarp, 0, s>>>(bv, q, s32, (int)n_reads, pieces, sc);
   }
   NA_CUDA(cudaGetLastError());
   // rescue tiers on the spill lists, with the library's own kernels
