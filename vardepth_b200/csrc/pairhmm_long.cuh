@@ -51,6 +51,7 @@
 // tall strip in lockstep, with one boost per warp and strip.
 #pragma once
 #include "pairhmm_kernel.cuh"
+#include "pairhmm_wait.h"
 
 namespace vd {
 
@@ -63,7 +64,6 @@ namespace vd {
 __host__ __device__ constexpr int long_max_bits(int rows) { return rows * 15 / 4; }
 constexpr int kLongTop = 100;             // a lane's bound for the coming steps, binary orders
 constexpr int kLongNone = -(1 << 28);     // exponent of "nothing there"
-constexpr long long kLongSpins = 1ll << 25;  // polls of one wait before it gives up (tens of seconds)
 
 // VD_LONG_BLOCK: runs of one tall strip before a half gives up, the window its
 // warps' bottoms must end in (cells a few dozen binary orders below a bottom's
@@ -154,29 +154,24 @@ __device__ __forceinline__ void st_release(unsigned long long* p, unsigned long 
   asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
 
-// A task's word: boundary blocks published so far (all of them: the task is
-// done), which halves left the range, and the buffer its boundary is in.
-__device__ __forceinline__ int task_blocks(unsigned long long v) { return (int)(v & 0x3fffffffull); }
-__device__ __forceinline__ unsigned task_fail(unsigned long long v) { return (unsigned)(v >> 30) & 3u; }
-__device__ __forceinline__ int task_buffer(unsigned long long v) { return (int)(v >> 32); }
-
-// Waits until the task behind `p` has published `need` blocks; returns its
-// word.  Every lane polls (one broadcast load).  After kLongSpins polls, or
-// once another wait has given up, the error flag is set and ok is false.
+// Waits until the task behind `p` has published `need` blocks; returns its word
+// (wait_word; the same in every lane).
+struct TaskWarp {
+  const unsigned long long* word;
+  int* error_flag;
+  __device__ __forceinline__ unsigned long long load() const { return ld_acquire(word); }
+  __device__ __forceinline__ bool stopped() const { return *(volatile int*)error_flag != 0; }
+  __device__ __forceinline__ void give_up() const { atomicExch(error_flag, 2); }
+  __device__ __forceinline__ void pause() const { __nanosleep(64); }
+  __device__ __forceinline__ unsigned long long from_leader(unsigned long long v) const {
+    v = __shfl_sync(0xffffffffu, v, 0);
+    __syncwarp();  // (the other lanes' reads of the boundary come after the leader's acquire)
+    return v;
+  }
+};
 __device__ __forceinline__ unsigned long long wait_task(const unsigned long long* p, int need, int* error_flag,
                                                         bool& ok) {
-  unsigned long long v = ld_acquire(p);
-  for (long long spin = 0; task_blocks(v) < need; ++spin) {
-    if (spin >= kLongSpins || ((spin & 1023) == 1023 && *(volatile int*)error_flag != 0)) {
-      atomicExch(error_flag, 2);
-      ok = false;
-      break;
-    }
-    __nanosleep(64);
-    v = ld_acquire(p);
-  }
-  ok = __all_sync(0xffffffffu, ok);
-  return v;
+  return wait_word(TaskWarp{p, error_flag}, need, ok);
 }
 
 // exponent of a non-negative float, kLongNone below the normal range
