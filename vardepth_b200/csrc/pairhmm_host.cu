@@ -266,6 +266,12 @@ struct vd_engine {
     vd_plan* pl = nullptr;
     bool busy = false;
     bool deferred = false;               // its rescue tiers wait for the counters
+    // nothing of the slot in flight, and nothing of it left to finish
+    void drain() {
+      if (stream) cudaStreamSynchronize(stream);
+      side.synchronize();
+      busy = deferred = false;
+    }
   };
   Slot slots[2];
 };
@@ -1703,6 +1709,17 @@ int vd_forward(vd_engine* e, const vd_batch* b, const vd_params* p, double* out,
     return VD_OK;
   };
 
+  // Every return leaves both slots idle: a chunk of a call that ended with an error
+  // must not be finished by a later call, whose output it does not belong to, nor
+  // copy into this call's output after the return.
+  struct Drain {
+    vd_engine* e;
+    bool armed = true;
+    ~Drain() {
+      if (armed) for (vd_engine::Slot& sl : e->slots) sl.drain();
+    }
+  } drain{e};
+
   int64_t u = 0, chunk_index = 0;
   // The kernels of a chunk wait for all kernels of the previous chunk (its
   // copies do not): FP32 kernels of two chunks sharing the SMs run different
@@ -1769,6 +1786,7 @@ int vd_forward(vd_engine* e, const vd_batch* b, const vd_params* p, double* out,
   // drain in submission order
   if ((rc = finish(e->slots[chunk_index & 1]))) return rc;
   if ((rc = finish(e->slots[(chunk_index + 1) & 1]))) return rc;
+  drain.armed = false;
   s.total_ms = now_ms() - t0;
   if (st) *st = s;
   return VD_OK;
@@ -1777,7 +1795,7 @@ int vd_forward(vd_engine* e, const vd_batch* b, const vd_params* p, double* out,
 namespace {
 // The whole batch as one chunk in a slot (ignoring the memory budget), its tiers
 // and the copy of their counters enqueued on the slot's stream.  The engine's lock
-// is held and the slot is idle.
+// is held and the slot is idle (every call that uses one drains it).
 int enqueue_whole(vd_engine* e, const vd_batch* b, const vd_params* p, vd_engine::Slot& sl, vd_stats* s) {
   int rc = ensure_tables(e, p);
   if (rc) return rc;
@@ -2223,7 +2241,7 @@ int vd_region_genotypes(vd_engine* e, const vd_batch* b, const vd_params* p, con
       vd_engine* e;
       vd_engine::Slot& sl;
       ~Drain() {
-        if (sl.stream) cudaStreamSynchronize(sl.stream);
+        sl.drain();
         if (sl.arena.bytes > e->budget) sl.arena.release();  // (this call ignores the memory budget)
       }
     } drain{e, sl};
