@@ -518,7 +518,7 @@ def main():
                            "descent, 1% threshold; a choice other than the default is kept only if one "
                            "captured run of the whole batch confirms it"}
 
-    # ---- the warp-per-pair / block-per-pair split on a batch of few long pairs ----
+    # ---- the two long-read paths on a batch of few long pairs ----
     split = None
     if args.workload == "mixed_length_regions" and world == 1:
         rl = np.diff(w.read_off)
@@ -533,8 +533,7 @@ def main():
             split = {"batch": f"one region with {len(one.read_off) - 1} reads of up to {int(longest[g])} bases",
                      "pairs": one.pairs(), "cells": one.cells(),
                      "kernel_ms": {}}
-            for name, mode in (("warp", native.VD_LONG_WARP), ("block", native.VD_LONG_BLOCK),
-                               ("single", native.VD_LONG_SINGLE)):
+            for name, mode in (("warp", native.VD_LONG_WARP), ("single", native.VD_LONG_SINGLE)):
                 engine.set_tuning(**dict(saved, long_mode=mode))
                 p1 = engine.plan(op, params)
                 p1.run()

@@ -145,9 +145,7 @@ typedef struct vd_tuning {
   int long_mode;        /* reads longer than one strip, FP32 semiglobal: VD_LONG_WARP (default) runs a
                            read against two haplotypes at a time, a warp per strip, the strips of
                            a pair side by side, lanes scaled by powers of two;
-                           VD_LONG_BLOCK the same items on a block per item, whose 4 warps split
-                           each strip (4x shorter latency per pair, for batches of few long
-                           pairs); VD_LONG_SINGLE the single-read kernel (strips renormalised
+                           VD_LONG_BLOCK the same with two haplotypes to an item; VD_LONG_SINGLE the single-read kernel (strips renormalised
                            exactly, error-rich reads then rescued by the drift tier) */
   int pair_split;       /* two-read items with at least this many rows per lane (6, the default, or 7)
                            run on the 12-warp-per-SM kernel (168 registers), fewer rows on the
@@ -155,7 +153,7 @@ typedef struct vd_tuning {
   int long_group;       /* VD_LONG_WARP: haplotypes per long-read item, 1..8 (0 = 8), run two at
                            a time (an odd one alone).  It sets which haplotypes share a warp and
                            the order of the work; a pair's likelihood does not depend on it.
-                           VD_LONG_BLOCK items hold two haplotypes. */
+                           VD_LONG_BLOCK items hold two haplotypes whatever it is. */
   int reserved[1];      /* must be zero */
 } vd_tuning;
 enum { VD_LONG_WARP = 0, VD_LONG_SINGLE = 1, VD_LONG_BLOCK = 2 };

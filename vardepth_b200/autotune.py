@@ -19,10 +19,9 @@ lays out the work list:
   the 31-step wavefront ramp less often);
 * ``long_mode``  how reads longer than one strip run: a read against two
   haplotypes at a time, a warp per strip with the strips of a pair side by
-  side (``VD_LONG_WARP``), on a whole CTA whose warps split each tall strip in
-  lockstep (``VD_LONG_BLOCK``), or one pair per warp in the single-read kernel
-  with exact strip renormalisation and the drift tier behind it
-  (``VD_LONG_SINGLE``);
+  side (``VD_LONG_WARP``; ``VD_LONG_BLOCK`` is the same kernel and is not
+  tried), or one pair per warp in the single-read kernel with exact strip
+  renormalisation and the drift tier behind it (``VD_LONG_SINGLE``);
 * ``long_group``  haplotypes per item of a long read: which of them share a
   warp, and the order of the work.  It is not searched: every strip is its
   own task, so the grouping hardly matters.
@@ -46,7 +45,7 @@ DEFAULT = {"long_read_rows": 256, "pair_mask": 0x1FE, "max_item_columns": 0, "lo
            "pair_split": 6, "long_group": native.LONG_GROUP_MAX}
 SPACE = {
     "pair_split": [6, 7],
-    "long_mode": [native.VD_LONG_WARP, native.VD_LONG_BLOCK, native.VD_LONG_SINGLE],
+    "long_mode": [native.VD_LONG_WARP, native.VD_LONG_SINGLE],
     "long_read_rows": [256, 128, 64],
     "pair_mask": [0x1FE, 0x1F0, 0],
     "max_item_columns": [0, 16384, 4096],

@@ -220,7 +220,7 @@ struct vd_engine {
   int grid[2][2] = {{0, 0}, {0, 0}};  // [f64][anchored] blocks
   int grid_pair[2][2] = {{0, 0}, {0, 0}};  // blocks of the two-read kernels [split == 7][wide]
   int grid_drift = 0;                 // blocks of the drift tier (no more than grid[0][0])
-  int grid_long[2][2] = {{0, 0}, {0, 0}};  // blocks of the long-read kernels [block][R == 8] (<= grid[0][0])
+  int grid_long[2] = {0, 0};          // blocks of the long-read kernels [R == 8] (<= grid[0][0])
   int grid_grad[2] = {0, 0};          // blocks of the gradient kernel [f64]
   int grid_grad_pair[2] = {0, 0};     // blocks of the two-pair gradient kernels [wide]
   vd_tuning tuning{256, 0x1fe, 0, 0, VD_LONG_WARP, 6, kLongGroupMax, {0}};  // vd_engine_set_tuning
@@ -363,7 +363,6 @@ int64_t batch_outputs(const vd_batch* b) {
 struct BuildOpts {
   int long_R = kMaxR;              // rows per lane of reads longer than one 256-row strip
   bool long_warp = true;           // such reads (FP32 semiglobal) run a read against two haplotypes per item
-  bool long_block = false;         // ... on a block per item (the CTA's warps split each strip)
   int long_group = kLongGroupMax;  // haplotypes per warp item of such a read
   int pair_split = 6;              // two-read items with this many rows per lane or more: 12-warp kernel
   int pair_mask = 0x1fe;           // bit R: two reads of R rows per lane may share a warp
@@ -380,9 +379,9 @@ int rows_per_lane(int n, int long_R = kMaxR) {
 
 // Rows per lane of a long read: as many strips as the strip height asks for,
 // of the fewest rows that hold the read (a 300-base read takes two strips of
-// 160 rows rather than of 256).  The block kernel and 128-row strips keep theirs.
+// 160 rows rather than of 256).  128-row strips keep theirs.
 int long_rows(int n, const BuildOpts& bo) {
-  if (bo.long_block || bo.long_R != kMaxR) return bo.long_R;
+  if (bo.long_R != kMaxR) return bo.long_R;
   const int strips = (n + kStripRows - 1) / kStripRows;
   return (n + kWarp * strips - 1) / (kWarp * strips);
 }
@@ -394,8 +393,8 @@ BuildOpts build_opts(const vd_engine* e) {
   bo.max_stream = e->tuning.max_item_columns > 0 ? (int64_t)e->tuning.max_item_columns : (int64_t)1 << 30;
   bo.long_warp = (e->tuning.long_mode == VD_LONG_WARP || e->tuning.long_mode == VD_LONG_BLOCK) &&
                  (bo.long_R == 8 || bo.long_R == 4);
-  bo.long_block = e->tuning.long_mode == VD_LONG_BLOCK;
-  bo.long_group = bo.long_block ? 2 : e->tuning.long_group > 0 ? e->tuning.long_group : kLongGroupMax;
+  // (VD_LONG_BLOCK names the same kernel with two haplotypes to an item)
+  bo.long_group = e->tuning.long_mode == VD_LONG_BLOCK ? 2 : e->tuning.long_group > 0 ? e->tuning.long_group : kLongGroupMax;
   bo.pair_split = e->tuning.pair_split == 7 ? 7 : 6;
   return bo;
 }
@@ -475,7 +474,6 @@ struct HostChunk {
   int pair_split = 6;              // rows per lane from which two-read items run at 12 warps per SM
   int64_t n_long = 0;              // the items after them: long reads, two haplotypes per item
   int long_R = kMaxR;              // rows per lane of those, at most
-  bool long_block = false;         // and their kernel: block per item (else a warp per strip of a pair)
   bool strip_singles = false;      // single-read items with reads longer than a strip beside them
   std::vector<int64_t> long_off;   // first task (strip of a pair) of each, and the total (not block)
 };
@@ -661,7 +659,6 @@ void build_region_chunk(const vd_batch* b, int64_t g0, int64_t g1, const TableSe
   const bool fp32 = pair_reads;  // mixed precision: the FP32 kernels run the primary tier
   if (plain) pair_reads = false;
   c.long_R = bo.long_R;
-  c.long_block = bo.long_block;
   c.ra = b->region_read_off[g0];
   c.rb = b->region_read_off[g1];
   c.ha = b->region_hap_off[g0];
@@ -846,7 +843,7 @@ void build_region_chunk(const vd_batch* b, int64_t g0, int64_t g1, const TableSe
   c.n_long = (int64_t)(lend - mid);
   c.strip_singles = c.n_long > 0 && std::any_of(lend, c.items.end(), [](const WorkItem& w) { return (w.code & 512) != 0; });
   c.long_off.clear();
-  if (c.n_long > 0 && !c.long_block) {
+  if (c.n_long > 0) {
     c.long_off.resize((size_t)c.n_long + 1);
     int64_t tasks = 0;
     for (int64_t k = 0; k < c.n_long; ++k) {
@@ -1183,8 +1180,7 @@ int enqueue_tiers(vd_plan* pl, int* launches, bool capturing = false, Tiers whic
       ql.long_words = (unsigned long long*)(d + L.o_lword);
       ql.long_exp_off = pl->chunk.max_hap + 1;
       const int R = pl->chunk.long_R;
-      const bool blk = pl->chunk.long_block;
-      err = launch_long_f32(R, blk, bv, ql, &dt->f32, ht->s32d, e->grid_long[blk ? 1 : 0][R == 8 ? 1 : 0], pl->side->s[0]);
+      err = launch_long_f32(R, bv, ql, &dt->f32, ht->s32d, e->grid_long[R == 8 ? 1 : 0], pl->side->s[0]);
       if (err != cudaSuccess) return cuda_fail(err, "long-read tier launch");
       ++n;
       VD_CUDA(cudaEventRecord(pl->side->join[0], pl->side->s[0]));
@@ -1344,13 +1340,12 @@ int init_engine_grids(vd_engine* e) {
   if (err != cudaSuccess) return cuda_fail(err, "occupancy query");
   // its warps index the strip scratch, which is sized by the largest grid
   e->grid_drift = std::min(std::max(1, bps) * e->sm_count, e->grid[0][0]);
-  for (int blk = 0; blk < 2; ++blk)
-    for (int k = 0; k < 2; ++k) {
-      bps = 0;
-      err = occupancy_long_f32(k ? 8 : 4, blk != 0, &bps);
-      if (err != cudaSuccess) return cuda_fail(err, "occupancy query");
-      e->grid_long[blk][k] = std::min(std::max(1, bps) * e->sm_count, e->grid[0][0]);
-    }
+  for (int k = 0; k < 2; ++k) {
+    bps = 0;
+    err = occupancy_long_f32(k ? 8 : 4, &bps);
+    if (err != cudaSuccess) return cuda_fail(err, "occupancy query");
+    e->grid_long[k] = std::min(std::max(1, bps) * e->sm_count, e->grid[0][0]);
+  }
   for (int f = 0; f < 2; ++f) {
     bps = 0;
     err = occupancy_grad(f != 0, &bps);
@@ -1372,7 +1367,7 @@ int64_t max_grid_warps(const vd_engine* e) {
 
 // warps of the kernel a chunk's long reads run on
 int64_t long_warps(const vd_engine* e, const HostChunk& c) {
-  return (int64_t)e->grid_long[c.long_block ? 1 : 0][c.long_R == kMaxR ? 1 : 0] * kWarpsPerBlock;
+  return (int64_t)e->grid_long[c.long_R == kMaxR ? 1 : 0] * kWarpsPerBlock;
 }
 
 std::mutex g_default_mu;
@@ -1612,7 +1607,7 @@ int vd_forward(vd_engine* e, const vd_batch* b, const vd_params* p, double* out,
   BuildOpts lbo = build_opts(e);
   lbo.item_limit = batch_item_limit(e, b, p);
   int64_t long_items = 0;
-  if (lbo.long_warp && !lbo.long_block && p->precision != VD_PRECISION_FLOAT64 && !p->anchored) {
+  if (lbo.long_warp && p->precision != VD_PRECISION_FLOAT64 && !p->anchored) {
     auto long_reads = [&](int64_t r0, int64_t r1) {
       int64_t k = 0;
       for (int64_t r = r0; r < r1; ++r) k += (b->read_off[r + 1] - b->read_off[r]) > kStripRows;
@@ -1632,7 +1627,7 @@ int vd_forward(vd_engine* e, const vd_batch* b, const vd_params* p, double* out,
   const int64_t pipeline_cells = (int64_t)(e->tuning.pipeline_gcells > 0 ? e->tuning.pipeline_gcells : 300) * 1'000'000'000LL;
   int64_t n_pipe = std::max<int64_t>(1, std::min<int64_t>(8, total_cells / pipeline_cells));
   if (long_items > 0) {
-    const int64_t long_warps = (int64_t)e->grid_long[0][lbo.long_R == 8 ? 1 : 0] * kWarpsPerBlock;
+    const int64_t long_warps = (int64_t)e->grid_long[lbo.long_R == 8 ? 1 : 0] * kWarpsPerBlock;
     n_pipe = std::max<int64_t>(1, std::min<int64_t>(n_pipe, long_items / (kLongItemsPerWarp * std::max<int64_t>(1, long_warps))));
   }
   const int64_t chunk_cells = n_pipe > 1 ? (total_cells + n_pipe - 1) / n_pipe : INT64_MAX;
@@ -1643,7 +1638,7 @@ int vd_forward(vd_engine* e, const vd_batch* b, const vd_params* p, double* out,
   for (int64_t r = 0; r < b->n_reads; ++r) max_read = std::max<int64_t>(max_read, b->read_off[r + 1] - b->read_off[r]);
   const int64_t scratch_warps = max_read + p->anchored > kStripRows ? warps : std::min<int64_t>(warps, (int64_t)kRobustBlocks * kWarpsPerBlock);
   // (two boundary buffers per warp of the long-read kernel where it runs)
-  const int64_t long_w = (int64_t)e->grid_long[lbo.long_block ? 1 : 0][lbo.long_R == kMaxR ? 1 : 0] * kWarpsPerBlock;
+  const int64_t long_w = (int64_t)e->grid_long[lbo.long_R == kMaxR ? 1 : 0] * kWarpsPerBlock;
   fixed += std::max((max_hap + 1) * scratch_warps, max_read > kStripRows ? 2 * long_buffer_records(max_hap) * long_w : 0) *
                (int64_t)sizeof(double2) +
            64 * 1024;
