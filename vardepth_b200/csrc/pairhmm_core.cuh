@@ -31,6 +31,7 @@
 //   ln Z = ln Zs - ln C_0 + sum_i ln N_i - E ln 2,   N_i = 1/f_i,
 // E being the sum of the power-of-two strip renormalisations.
 #pragma once
+#include <cmath>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -93,6 +94,13 @@ struct Scalars {
   T final_floor;             // below this the final scaled sum counts as underflowed
   int target_log2;           // strip boundary maxima are renormalised to 2^target
 };
+
+// The same for the robust tier, which has no tier behind it: what 32 rows can lose
+// (43 bits each) stays inside its strips.
+inline Scalars<double> robust_scalars(Scalars<double> s) {
+  s.strip_floor = ldexp(1.0, -800);
+  return s;
+}
 
 // Device-side view of one batch.
 struct BatchView {

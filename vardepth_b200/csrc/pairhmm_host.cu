@@ -132,7 +132,10 @@ void build_tables(double g, double x, const double* offsets, TableSet* ts) {
   ts->s32d.target_log2 = 0;
   ts->s64.k2 = k2; ts->s64.x = x; ts->s64.gfin = g;
   ts->s64.c = std::ldexp(1.0, 600); ts->s64.ln_c = 600.0 * std::log(2.0);
-  ts->s64.strip_floor = std::ldexp(1.0, -800); ts->s64.final_floor = std::ldexp(1.0, -900);
+  // a boundary keeps what lies up to 1,024 binary orders below its largest cell, as
+  // rows divided by their maximum do; a strip that loses more than 650 bits runs again
+  // in strips of 32 rows
+  ts->s64.strip_floor = std::ldexp(1.0, -50); ts->s64.final_floor = std::ldexp(1.0, -900);
   ts->s64.strip_ceil = HUGE_VAL;
   ts->s64.target_log2 = 600;
 }
@@ -1267,7 +1270,7 @@ int enqueue_tiers(vd_plan* pl, int* launches, bool capturing = false, Tiers whic
     q2.spill_count = nullptr;
     q2.spill_cap = 0;
     const int robust_grid = pl->chunk.any_strip ? e->grid[1][anch] : std::min(e->grid[1][anch], kRobustBlocks);
-    err = launch_f64(anch, rv, q2, &dt->f64, ht->s64, 2, robust_grid, pl->stream);
+    err = launch_f64(anch, rv, q2, &dt->f64, robust_scalars(ht->s64), 2, robust_grid, pl->stream);
     if (err != cudaSuccess) return cuda_fail(err, "robust tier launch");
     ++n;
   } else {

@@ -539,7 +539,7 @@ extern "C" int vd_forward_region_noalloc(int device, const unsigned char* read_b
   q2.spill = nullptr;
   q2.spill_count = nullptr;
   q2.spill_cap = 0;
-  NA_CUDA(launch_f64(anch, rv, q2, t64, s64, 2, std::min(d.rescue[anch], kNaRobustBlocks), s));
+  NA_CUDA(launch_f64(anch, rv, q2, t64, robust_scalars(s64), 2, std::min(d.rescue[anch], kNaRobustBlocks), s));
   // length checks and the overflow flag come back with the stream
   unsigned long long h[16];
   NA_CUDA(cudaMemcpyAsync(h, sc + kOffCnt, sizeof(h), cudaMemcpyDeviceToHost, s));
