@@ -88,7 +88,7 @@ struct TableSet {
   Tables<double> f64;
   Scalars<float> s32;
   Scalars<double> s64;
-  Scalars<float> s32d;  // the drift tier: row 0 = 1, strips brought to 2^0, window 2^-60 .. 2^60
+  Scalars<float> s32d;  // the long-read kernel and the drift tier: row 0 = 1
 };
 
 // Per-quality factors of the scaled recurrence (pairhmm_core.cuh).  The error
@@ -120,23 +120,16 @@ void build_tables(double g, double x, const double* offsets, TableSet* ts) {
   // sum >= 2^-80 keeps the dominant cells normal (>= 2^-93 after m+1 <= 2^13 terms)
   ts->s32.c = std::ldexp(1.0f, 120); ts->s32.ln_c = 120.0 * std::log(2.0);
   ts->s32.strip_floor = std::ldexp(1.0f, -40); ts->s32.final_floor = std::ldexp(1.0f, -80);
-  ts->s32.strip_ceil = HUGE_VALF;
   ts->s32.target_log2 = 120;
-  // the drift tier keeps every strip's bottom near 2^0 with per-row boosts, so
-  // it starts there and leaves 60 binary orders either side for what the
-  // boosts do not cancel
+  // the long-read kernel and the drift tier choose their own exponents
   ts->s32d = ts->s32;
   ts->s32d.c = 1.0f; ts->s32d.ln_c = 0.0;
-  ts->s32d.strip_floor = std::ldexp(1.0f, -60); ts->s32d.strip_ceil = std::ldexp(1.0f, 60);
-  ts->s32d.final_floor = std::ldexp(1.0f, -60);
-  ts->s32d.target_log2 = 0;
   ts->s64.k2 = k2; ts->s64.x = x; ts->s64.gfin = g;
   ts->s64.c = std::ldexp(1.0, 600); ts->s64.ln_c = 600.0 * std::log(2.0);
   // a boundary keeps what lies up to 1,024 binary orders below its largest cell, as
   // rows divided by their maximum do; a strip that loses more than 650 bits runs again
   // in strips of 32 rows
   ts->s64.strip_floor = std::ldexp(1.0, -50); ts->s64.final_floor = std::ldexp(1.0, -900);
-  ts->s64.strip_ceil = HUGE_VAL;
   ts->s64.target_log2 = 600;
 }
 
@@ -222,7 +215,7 @@ struct vd_engine {
   std::mutex mu;
   int grid[2][2] = {{0, 0}, {0, 0}};  // [f64][anchored] blocks
   int grid_pair[2][2] = {{0, 0}, {0, 0}};  // blocks of the two-read kernels [split == 7][wide]
-  int grid_drift = 0;                 // blocks of the drift tier (no more than grid[0][0])
+  int grid_drift = 0;                 // blocks of the drift tier
   int grid_long[2] = {0, 0};          // blocks of the long-read kernels [R == 8] (<= grid[0][0])
   int grid_grad[2] = {0, 0};          // blocks of the gradient kernel [f64]
   int grid_grad_pair[2] = {0, 0};     // blocks of the two-pair gradient kernels [wide]
@@ -935,16 +928,29 @@ void build_pair_chunk(const vd_batch* b, const PairGroups& pg, int64_t ra, int64
   if (!plain) order_items(c.items, cost);
 }
 
+int64_t max_grid_warps(const vd_engine* e) {
+  int g = 0;
+  for (int f = 0; f < 2; ++f) for (int a = 0; a < 2; ++a) g = std::max(g, e->grid[f][a]);
+  return (int64_t)g * kWarpsPerBlock;
+}
+
+// warps of the kernel a chunk's long reads run on
+int64_t long_warps(const vd_engine* e, const HostChunk& c) {
+  return (int64_t)e->grid_long[c.long_R == kMaxR ? 1 : 0] * kWarpsPerBlock;
+}
+
 // Device bytes a chunk needs (inputs, lists, outputs, rescue lists, scratch).
 struct Layout {
   size_t o_rb, o_rq, o_roff, o_rcode, o_hb, o_hoff, o_hsel, o_osel, o_hord, o_hshare, o_items, o_loff, o_out, o_sp1,
       o_sp2, o_cnt, o_lword, o_scratch, o_long, total;
   int64_t scratch_stride;  // double2 records per warp slot
-  int64_t long_stride;     // the same of the long-read kernels (two boundary buffers)
-  int64_t warps;
+  int64_t long_stride;     // the same of the long-read kernel (two boundary buffers)
+  int64_t drift_stride;    // the same of the drift tier (0: reads of one strip only)
+  int drift_blocks;        // blocks of the drift tier the scratch holds
 };
 
-Layout layout_for(const HostChunk& c, const vd_batch* b, int64_t warps, int64_t long_warps) {
+Layout layout_for(const vd_engine* e, const HostChunk& c) {
+  const int64_t warps = max_grid_warps(e), warps_long = long_warps(e, c);
   Layout L{};
   size_t off = 0;
   auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + std::max<size_t>(bytes, 1), 256); return o; };
@@ -974,12 +980,16 @@ Layout layout_for(const HostChunk& c, const vd_batch* b, int64_t warps, int64_t 
   // reads with Phred 0 or 1 bases), needs its own.
   L.scratch_stride = c.any_long ? (int64_t)c.max_hap + 1 : 0;
   L.long_stride = c.n_long > 0 ? 2 * long_buffer_records(c.max_hap) : 0;
-  L.warps = c.any_strip ? warps : std::min<int64_t>(warps, (int64_t)kRobustBlocks * kWarpsPerBlock);
-  const int64_t own = std::max<int64_t>(1, L.scratch_stride) * warps, shared = L.long_stride * long_warps;
+  const int64_t own = std::max<int64_t>(1, L.scratch_stride) * warps, shared = L.long_stride * warps_long;
   L.o_scratch = take((size_t)(c.strip_singles ? own : std::max(own, shared)) * sizeof(double2));
   L.o_long = c.strip_singles ? take((size_t)shared * sizeof(double2)) : L.o_scratch;
+  // the drift tier runs after both and takes as many blocks as the larger holds
+  L.drift_stride = c.any_strip ? 2 * long_buffer_records(c.max_hap) : 0;
+  L.drift_blocks = e->grid_drift;
+  if (c.any_strip)
+    L.drift_blocks = (int)std::min<int64_t>(L.drift_blocks, (c.strip_singles ? own : std::max(own, shared)) /
+                                                                (L.drift_stride * kWarpsPerBlock));
   L.total = off;
-  (void)b;
   return L;
 }
 
@@ -1241,8 +1251,9 @@ int enqueue_tiers(vd_plan* pl, int* launches, bool capturing = false, Tiers whic
       qd.head = cnt + 9;
       qd.spill = (RescueEntry*)(d + L.o_sp2);
       qd.spill_count = cnt + 4;
-      qd.scratch_stride = 2 * L.scratch_stride;  // two float2 boundaries in each warp's double2 slot
-      err = launch_drift_f32(rv, qd, &dt->f32, ht->s32d, e->grid_drift, pl->stream);
+      qd.scratch_stride = L.drift_stride;
+      qd.long_exp_off = pl->chunk.max_hap + 1;
+      err = launch_drift_f32(rv, qd, &dt->f32, ht->s32d, L.drift_blocks, pl->stream);
       if (err != cudaSuccess) return cuda_fail(err, "drift tier launch");
       ++n;
     }
@@ -1341,8 +1352,7 @@ int init_engine_grids(vd_engine* e) {
   bps = 0;
   err = occupancy_drift_f32(&bps);
   if (err != cudaSuccess) return cuda_fail(err, "occupancy query");
-  // its warps index the strip scratch, which is sized by the largest grid
-  e->grid_drift = std::min(std::max(1, bps) * e->sm_count, e->grid[0][0]);
+  e->grid_drift = std::max(1, bps) * e->sm_count;
   for (int k = 0; k < 2; ++k) {
     bps = 0;
     err = occupancy_long_f32(k ? 8 : 4, &bps);
@@ -1360,17 +1370,6 @@ int init_engine_grids(vd_engine* e) {
     e->grid_grad_pair[f] = std::max(1, bps) * e->sm_count;
   }
   return VD_OK;
-}
-
-int64_t max_grid_warps(const vd_engine* e) {
-  int g = 0;
-  for (int f = 0; f < 2; ++f) for (int a = 0; a < 2; ++a) g = std::max(g, e->grid[f][a]);
-  return (int64_t)g * kWarpsPerBlock;
-}
-
-// warps of the kernel a chunk's long reads run on
-int64_t long_warps(const vd_engine* e, const HostChunk& c) {
-  return (int64_t)e->grid_long[c.long_R == kMaxR ? 1 : 0] * kWarpsPerBlock;
 }
 
 std::mutex g_default_mu;
@@ -1756,7 +1755,7 @@ int vd_forward(vd_engine* e, const vd_batch* b, const vd_params* p, double* out,
     else build_region_chunk(b, u, u_end, e->htab, offsets, p->anchored != 0, p->precision == VD_PRECISION_MIXED,
                             pl.chunk, plain, bo);
     HostChunk& c = pl.chunk;
-    pl.L = layout_for(c, b, warps, long_warps(e, c));
+    pl.L = layout_for(e, c);
     s.host_ms += now_ms() - th;
     if ((rc = sl.arena.reserve(pl.L.total))) return rc;
     pl.base = (char*)sl.arena.p;
@@ -1814,7 +1813,7 @@ int enqueue_whole(vd_engine* e, const vd_batch* b, const vd_params* p, vd_engine
   build_region_chunk(b, 0, b->n_regions, e->htab, p->quality_offsets != nullptr, p->anchored != 0,
                      p->precision == VD_PRECISION_MIXED, pl.chunk, p->schedule == VD_SCHEDULE_PLAIN, bo);
   HostChunk& c = pl.chunk;
-  pl.L = layout_for(c, b, max_grid_warps(e), long_warps(e, c));
+  pl.L = layout_for(e, c);
   s->host_ms += now_ms() - th;
   if ((rc = sl.arena.reserve(pl.L.total))) return rc;
   pl.base = (char*)sl.arena.p;
@@ -1868,7 +1867,7 @@ int vd_plan_create(vd_engine* e, const vd_batch* b, const vd_params* p, vd_plan*
     build_region_chunk(b, 0, b->n_regions, e->htab, offsets, p->anchored != 0, p->precision == VD_PRECISION_MIXED,
                        pl->chunk, plain, bo);
   }
-  pl->L = layout_for(pl->chunk, b, max_grid_warps(e), long_warps(e, pl->chunk));
+  pl->L = layout_for(e, pl->chunk);
   if ((rc = pl->own.reserve(pl->L.total))) { delete pl; return rc; }
   pl->base = (char*)pl->own.p;
   if ((rc = upload_chunk(pl, b, nullptr))) { delete pl; return rc; }

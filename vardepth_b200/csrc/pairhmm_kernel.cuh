@@ -93,21 +93,9 @@ __device__ __forceinline__ void spill_pair(const QueueView& qv, int32_t read, in
 
 constexpr int kUnroll = 8;
 
-// The drift tier (FP32, semiglobal) rescores the pairs the primary tier
-// spilled.  Error-rich long reads lose more per strip
-// than the FP32 range holds (8% errors at reported Q30: about 1 bit per row),
-// so each row's constants are multiplied by an exact power of two 2^k_i that
-// cancels the decay: Bs bits per strip, spread over its rows.  Bs is measured
-// as the read goes (the next strip takes the decay left over at the bottom of
-// this one) and a strip whose bottom leaves the window [2^-60, 2^60) is run
-// again with Bs corrected by the measured exponent (its input boundary is kept
-// in the other half of the warp's scratch).  A read of one strip spilled
-// because its likelihood lies below the primary tier's range; its lanes each
-// take their own boost, measured lane by lane (a variant or a cluster of
-// errors concentrates the decay in a few rows).  What still fails goes to FP64.
-constexpr int kDriftTries = 6;
-// Reads of several strips need a gap-continuation probability of at least
-// this for FP32 to hold them (pairhmm_long.cuh); below it they go to FP64.
+// Reads of several strips, and pairs of the drift tier, need a gap-continuation
+// probability of at least this for FP32 to hold them (pairhmm_long.cuh); below
+// it they go to FP64.
 constexpr float kLongMinExt = 0.0025f;
 
 // Row layout of one read (lane L, register r of strip s holds row
@@ -126,7 +114,7 @@ constexpr uint32_t kNeverBase = 0x10000u;  // compares unequal to every base byt
 // for why): 20,000 single reads of 96 / 150 bases 3,285 / 3,166 -> 3,611 /
 // 3,582 GCUPS, in FP64 of 250 bases 1,814 -> 1,936 (a lone warp 140 -> 94 ns a
 // step; the called function spilled).
-template <typename T, int R, bool GEN, bool ANCH, bool DRIFT = false>
+template <typename T, int R, bool GEN, bool ANCH>
 __device__ __forceinline__ void process_item(const BatchView& bv, const QueueView& qv, const ItemRef& it,
                                           const Tables<T>* __restrict__ tb, const Scalars<T>& sc,
                                           const int lane, typename Vec2<T>::type* __restrict__ scratch) {
@@ -159,36 +147,24 @@ __device__ __forceinline__ void process_item(const BatchView& bv, const QueueVie
 
   const T A = tb->A[rqual[n - 1]];
   const T k2 = sc.k2, x = sc.x, c0 = sc.c, gfin = sc.gfin;
-  int E = 0;          // total power-of-two scaling: strip renormalisations (and the drift tier's row boosts)
+  int E = 0;          // total power-of-two scaling of the strip renormalisations
   bool fail = false;  // a strip boundary left the range
 
-  // drift tier: per-row power-of-two boosts, strips re-run when they leave the
-  // window; the scratch holds two boundaries (read one, write the other)
-  constexpr bool kCanDrift = DRIFT && std::is_same<T, float>::value && GEN && !ANCH;
-  constexpr bool drift = kCanDrift;
-  const long long half = drift ? qv.scratch_stride / 2 : qv.scratch_stride;
-  int strip_lg = 0;     // drift: exponent of the strip's bottom maximum (or +-1024: inf / zero)
-  double zkeep = 0.0;   // drift: the last strip's final sum, on lane 31
-  // drift, reads of one strip: each lane's own boost bits (spread over its read
-  // rows) and the maximum of its bottom row's u over the columns of the last run
-  bool lane_boost = false;
-  int kl_lane = 0;
-  T lmax_keep = T(0);
+  const long long half = qv.scratch_stride;
 
-  // One strip of rows (Bs: the drift tier's boost bits for the strip, else 0).
+  // One strip of rows.
   // FIRST and LAST are compile-time tags, so the steady loop carries no
   // per-step test of the strip position.  Returns false when the strip's
-  // bottom boundary left [strip_floor, strip_ceil).
-  auto run_strip = [&](auto first_tag, auto last_tag, const int strip, const int Bs) -> bool {
+  // bottom boundary fell below strip_floor.
+  auto run_strip = [&](auto first_tag, auto last_tag, const int strip) -> bool {
     constexpr bool FIRST = decltype(first_tag)::value;
     constexpr bool last = decltype(last_tag)::value;
     const bool lane0 = lane == 0;
     LaneRows<T, R, GEN> rw;
     const int row0 = strip * SR + lane * R - v;
-    // the boundary this strip reads and the one it writes
-    T2* const src = scratch + (drift ? (long long)(strip & 1) * half : 0ll);
-    T2* const dst = scratch + (drift ? (long long)((strip + 1) & 1) * half : 0ll);
-    const int ns = min(SR, n - strip * SR);  // read rows of the strip (drift: semiglobal, v = 0)
+    // the boundary this strip reads and overwrites with its own
+    T2* const src = scratch;
+    T2* const dst = scratch;
     int emu = -1;  // register of the anchored row-0 emulator in this lane
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -200,21 +176,6 @@ __device__ __forceinline__ void process_item(const BatchView& bv, const QueueVie
         if (GEN) rw.hit[r] = tb->hit[q];
         rw.K[r] = tb->K[q];
         rw.X[r] = (!ANCH && i == n - 1) ? A : tb->X[q];
-        if constexpr (kCanDrift) {
-          {
-            // row il of the strip gets k = floor((il+1) Bs / ns) - floor(il Bs / ns),
-            // or its share of the lane's own boost (the lane's read rows split it)
-            const int il = i - strip * SR;
-            const int lrows = min(R, n - lane * R);
-            const int kr = lane_boost ? (r + 1) * kl_lane / lrows - r * kl_lane / lrows
-                                      : (il + 1) * Bs / ns - il * Bs / ns;
-            const T f = pow2T(kr, T(0));
-            rw.miss[r] *= f;
-            rw.hit[r] *= f;
-            rw.K[r] *= f;
-            rw.X[r] *= f;
-          }
-        }
       } else {
         const bool emulator = ANCH && i == -1;
         if (emulator) emu = r;
@@ -235,7 +196,6 @@ __device__ __forceinline__ void process_item(const BatchView& bv, const QueueVie
     const uint8_t* hp = bv.hap_bases;  // hp[p] = haplotype base at stream position p
     T s_top = T(0), u_bot = T(0);
     T acc32 = T(0), cap = T(0), rmax = T(0), bmax = T(0);
-    T lmax = T(0);  // drift: maximum of this lane's bottom-row u
     double acc64 = 0.0;
 
     auto finalize = [&](int k) {
@@ -248,10 +208,6 @@ __device__ __forceinline__ void process_item(const BatchView& bv, const QueueVie
       // than 1e-300 below that row maximum
       const double Zc = ANCH ? fmax(Zs, 1e-300 * (double)rmax) : Zs;
       const double lnC0 = sc.ln_c + (ANCH ? 0.0 : log((double)(m + 1)));
-      if constexpr (drift) {
-        zkeep = Zs;  // checked (and written) once the strip is done
-        return;
-      }
       const bool ok = !fail && Zs >= (double)sc.final_floor && Zs < HUGE_VAL;
       if (ok || qv.spill == nullptr) {
         bv.out[o] = (Zc > 0.0 ? log(Zc) : -HUGE_VAL) - lnC0 + lnN - (double)E * kLn2;
@@ -354,9 +310,6 @@ __device__ __forceinline__ void process_item(const BatchView& bv, const QueueVie
       s_in = lane0 ? is : s_in;
       T tmu = T(0), tnu = T(0), tom = T(0);
       column<T, R, GEN, ANCH>(rw, hb, s_top, u_in, k2, x, u_bot, tmu, tnu, tom);
-      if constexpr (drift) {
-        if (active) lmax = maxT(lmax, u_bot);
-      }
       s_top = s_in;
       if (last) {
         accumulate(tmu, tnu, tom);
@@ -389,7 +342,6 @@ __device__ __forceinline__ void process_item(const BatchView& bv, const QueueVie
       s_in = lane0 ? is : s_in;
       T tmu = T(0), tnu = T(0), tom = T(0);
       column<T, R, GEN, ANCH>(rw, hb, s_top, u_in, k2, x, u_bot, tmu, tnu, tom);
-      if constexpr (drift) lmax = maxT(lmax, u_bot);
       s_top = s_in;
       if (last) {
         accumulate(tmu, tnu, tom);
@@ -431,21 +383,14 @@ __device__ __forceinline__ void process_item(const BatchView& bv, const QueueVie
       }
       S = Snext;
     }
-    if constexpr (drift) lmax_keep = lmax;
-
     if (!last) {
       // renormalise the boundary the next strip starts from: its maximum is
       // brought to 2^target by an exact power of two, applied as two factors
       // so that any exponent shift stays representable
       __syncwarp();
       const T bm = __shfl_sync(FULL, bmax, kWarp - 1);
-      if (!(bm >= sc.strip_floor) || !(bm < sc.strip_ceil)) {
-        // (1024: overflowed to inf or NaN, -1024: underflowed to zero)
-        strip_lg = (bm != bm || bm >= T(HUGE_VAL)) ? 1024 : (bm > T(0) ? ilogb(bm) : -1024);
-        return false;
-      }
-      strip_lg = ilogb(bm);
-      const int ks = sc.target_log2 - strip_lg;
+      if (!(bm >= sc.strip_floor) || !(bm < T(HUGE_VAL))) return false;
+      const int ks = sc.target_log2 - ilogb(bm);
       const int k1 = ks / 2;
       const T f1 = pow2T(k1, T(0)), f2 = pow2T(ks - k1, T(0));
       for (int p = lane; p < S - 1; p += kWarp) {
@@ -460,113 +405,12 @@ __device__ __forceinline__ void process_item(const BatchView& bv, const QueueVie
     return true;
   };
 
-  if constexpr (drift) {
-    // rescue entries carry one haplotype
-    bool ok = K == 1;
-    if (nstrips == 1) {
-      // a read of one strip: the primary tier (row 0 at 2^120) spilled it because
-      // its final sum fell below 2^-80, so it decays by more than 200 bits.  Each
-      // lane boosts its own read rows.  The first run spreads 232 bits (32 above
-      // that bound) evenly over the read; a run is kept when every lane's
-      // bottom-row maximum and the final sum lie in 2^-60 .. 2^60.  Otherwise
-      // each lane takes the decay it measured (its boost plus its input's
-      // exponent minus its bottom's), so the next run holds every lane near 2^0
-      // wherever the read's errors sit.  The first lane whose bottom under- or
-      // overflowed moves by the bound that shows (149 bits: a nonzero float would
-      // have been seen), and the lanes below it take the mean rate of the lanes
-      // above.
-      const int used = (n + R - 1) / R;  // lanes holding read rows
-      const int lrows = lane < used ? min(R, n - lane * R) : 0;
-      const int B0 = min(16 * n, 232);
-      lane_boost = true;
-      kl_lane = lane < used ? (lane * R + lrows) * B0 / n - (lane * R) * B0 / n : 0;
-      for (int attempt = 0; ok; ++attempt) {
-        run_strip(std::true_type{}, std::true_type{}, 0, 0);
-        const double z = __shfl_sync(FULL, zkeep, kWarp - 1);
-        const T lm = lmax_keep;
-        const int lgl = lane >= used ? 0 : (lm != lm || lm >= T(HUGE_VAL)) ? 1024 : (lm > T(0) ? ilogb(lm) : -1024);
-        const bool in_window = lgl >= -60 && lgl < 60;
-        if (__all_sync(FULL, in_window) && z >= (double)sc.final_floor && z < (double)sc.strip_ceil) break;
-        if (attempt + 1 == kDriftTries) { ok = false; break; }
-        int in = __shfl_up_sync(FULL, lgl, 1);
-        if (lane == 0) in = 0;  // row 0 (c = 1)
-        const bool measured = lgl > -1024 && lgl < 1024;
-        const unsigned bad = __ballot_sync(FULL, lane < used && !measured);
-        const int first_bad = bad ? __ffs(bad) - 1 : kWarp;
-        const bool valid = lane < used && lane < first_bad;
-        const int d = valid ? kl_lane + in - lgl : 0;
-        int sum_d = d, sum_r = valid ? lrows : 0;
-#pragma unroll
-        for (int o = 16; o; o >>= 1) {
-          sum_d += __shfl_xor_sync(FULL, sum_d, o);
-          sum_r += __shfl_xor_sync(FULL, sum_r, o);
-        }
-        int k = kl_lane;
-        if (valid) {
-          k = d;
-        } else if (lane < used) {
-          if (sum_r > 0) k = (int)((long long)sum_d * lrows / sum_r);
-          if (lane == first_bad) k = lgl == -1024 ? max(k, kl_lane + in + 149) : min(k, kl_lane + in - 128);
-        }
-        kl_lane = max(-24 * lrows, min(24 * lrows, k));
-      }
-      if (ok) {
-        E = kl_lane;
-#pragma unroll
-        for (int o = 16; o; o >>= 1) E += __shfl_xor_sync(FULL, E, o);
-      }
-    } else if (sc.x < (T)kLongMinExt) {
-      ok = false;
-    } else if constexpr (R == kMaxR || R == 4 || R == 2 || R == 1) {
-      int Bs = SR;  // first guess: one bit per row (the spilled reads lost more than 160 per strip)
-      for (int strip = 0; ok && strip < nstrips; ++strip) {
-        const int ns = min(SR, n - strip * SR);
-        for (int attempt = 0;; ++attempt) {
-          bool good;
-          if (strip == 0) {
-            good = run_strip(std::true_type{}, std::false_type{}, strip, Bs);
-          } else if (strip < nstrips - 1) {
-            good = run_strip(std::false_type{}, std::false_type{}, strip, Bs);
-          } else {
-            run_strip(std::false_type{}, std::true_type{}, strip, Bs);
-            const double z = __shfl_sync(FULL, zkeep, kWarp - 1);
-            good = z >= (double)sc.final_floor && z < (double)sc.strip_ceil;
-            strip_lg = (z != z || z >= HUGE_VAL) ? 1024 : (z > 0.0 ? ilogb(z) : -1024);
-          }
-          // bottom exponent above the target: the boosts were too strong
-          const int excess = strip_lg - sc.target_log2;
-          if (good) {
-            E += Bs;
-            if (strip + 1 < nstrips) {
-              // the next strip takes this one's rate plus what it left over
-              const int ns1 = min(SR, n - (strip + 1) * SR);
-              Bs = max(0, min(16 * ns1, (Bs - excess) * ns1 / ns));
-            }
-            break;
-          }
-          if (attempt + 1 == kDriftTries) {
-            ok = false;
-            break;
-          }
-          const int step = (strip_lg == 1024) ? -ns / 2 : (strip_lg == -1024) ? ns / 2 : -excess;
-          Bs = max(0, min(16 * ns, Bs + (step != 0 ? step : (excess > 0 ? -1 : 1))));
-        }
-      }
-    } else {
-      ok = false;  // no strip-mined variant at this R: the pair goes on to FP64
-    }
-    if (ok && lane == kWarp - 1) {
-      const int64_t h = hap_index(0);
-      const int m = (int)(bv.hap_off[h + 1] - bv.hap_off[h]);
-      bv.out[out_index(0)] = log(zkeep) - (sc.ln_c + log((double)(m + 1))) + lnN - (double)E * kLn2;
-    }
-    fail = !ok;
-  } else if (nstrips == 1) {
-    run_strip(std::true_type{}, std::true_type{}, 0, 0);
+  if (nstrips == 1) {
+    run_strip(std::true_type{}, std::true_type{}, 0);
   } else if constexpr (R == kMaxR || R == 4 || R == 2 || R == 1) {
-    bool ok = run_strip(std::true_type{}, std::false_type{}, 0, 0);
-    for (int strip = 1; ok && strip < nstrips - 1; ++strip) ok = run_strip(std::false_type{}, std::false_type{}, strip, 0);
-    if (ok) ok = run_strip(std::false_type{}, std::true_type{}, nstrips - 1, 0);
+    bool ok = run_strip(std::true_type{}, std::false_type{}, 0);
+    for (int strip = 1; ok && strip < nstrips - 1; ++strip) ok = run_strip(std::false_type{}, std::false_type{}, strip);
+    if (ok) ok = run_strip(std::false_type{}, std::true_type{}, nstrips - 1);
     fail = !ok;
   } else {
     fail = true;  // not reached: reads longer than one strip run with R = 8, 4 or 2 (1 in the robust tier)
@@ -1058,61 +902,6 @@ pairhmm_pair_kernel(const __grid_constant__ BatchView bv, const __grid_constant_
       VD_PCASE(1) VD_PCASE(2) VD_PCASE(3) VD_PCASE(4) VD_PCASE(5) VD_PCASE(6) VD_PCASE(7) VD_PCASE(8)
 #undef VD_PCASE
       default: break;
-    }
-  }
-}
-
-// The drift tier (FP32, semiglobal): the rescue list of the primary tier,
-// each entry in the two-sided emission form its boosted match factors need,
-// on its own kernel so the strip driver's state does not crowd the primary
-// kernel's registers (launched with 4 blocks per SM, 128 registers: 7% faster
-// on the mixed-length workload's long reads than 3 blocks at 162 registers without spills).
-// Reads of one strip run at their own rows per lane; longer reads whose rows
-// per lane have no strip-mined variant go on to FP64 unchanged.
-template <int kBlocks>
-__global__ void __launch_bounds__(kWarpsPerBlock * kWarp, kBlocks)
-pairhmm_drift_kernel(const __grid_constant__ BatchView bv, const __grid_constant__ QueueView qv,
-                     const Tables<float>* __restrict__ gtab, const __grid_constant__ Scalars<float> sc) {
-  if (*qv.count == 0) return;
-  __shared__ Tables<float> tab;
-  {
-    const int words = (int)(sizeof(Tables<float>) / sizeof(int));
-    const int* src = reinterpret_cast<const int*>(gtab);
-    int* dst = reinterpret_cast<int*>(&tab);
-    for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & (kWarp - 1);
-  const long long gw = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
-  float2* scratch = reinterpret_cast<float2*>(qv.scratch) + gw * qv.scratch_stride;
-  long long total = qv.n_items;
-  const long long c = (long long)*qv.count;
-  total = c < total ? c : total;
-  for (;;) {
-    unsigned long long i = 0;
-    if (lane == 0) i = atomicAdd(qv.head, 1ull);
-    i = __shfl_sync(0xffffffffu, i, 0);
-    if ((long long)i >= total) break;
-    const RescueEntry e = qv.entries[i];
-    ItemRef it;
-    it.tier = kDriftTier;
-    it.use_sel = false;
-    it.w.read = e.read;
-    it.w.nhap = 1;
-    it.w.hap_begin = e.hap;
-    it.w.out_begin = e.out;
-    it.w.read2 = -1;
-    it.w.out2_begin = 0;
-    it.w.code = bv.read_code[e.read];
-    switch (code_R(it.w.code)) {
-#define VD_DCASE(r) \
-      case r: process_item<float, r, true, false, true>(bv, qv, it, &tab, sc, lane, scratch); break;
-      VD_DCASE(1) VD_DCASE(2) VD_DCASE(3) VD_DCASE(4) VD_DCASE(5) VD_DCASE(6) VD_DCASE(7) VD_DCASE(8)
-#undef VD_DCASE
-      default:
-        if (lane == 0) spill_pair<float>(qv, e.read, e.hap, e.out);
-        __syncwarp();
-        break;
     }
   }
 }

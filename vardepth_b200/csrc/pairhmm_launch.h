@@ -15,7 +15,7 @@ cudaError_t occupancy_f64(bool anchored, int* blocks_per_sm);
 cudaError_t launch_pair_f32(bool wide, int split, const BatchView& bv, const QueueView& qv,
                             const Tables<float>* tab, const Scalars<float>& sc, int grid, cudaStream_t stream);
 cudaError_t occupancy_pair_f32(bool wide, int split, int* blocks_per_sm);
-// the drift tier (FP32 semiglobal rescue with per-row power-of-two boosts)
+// the drift tier (FP32 semiglobal rescue, per-lane power-of-two exponents)
 cudaError_t launch_drift_f32(const BatchView& bv, const QueueView& qv, const Tables<float>* tab,
                              const Scalars<float>& sc, int grid, cudaStream_t stream);
 cudaError_t occupancy_drift_f32(int* blocks_per_sm);

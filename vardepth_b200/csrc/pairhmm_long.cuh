@@ -62,18 +62,19 @@ __host__ __device__ constexpr int long_max_bits(int rows) { return rows * 15 / 4
 constexpr int kLongTop = 100;             // a lane's bound for the coming steps, binary orders
 constexpr int kLongNone = -(1 << 28);     // exponent of "nothing there"
 
-template <int R>
+template <int R, bool GEN = false>
 struct LongRows {
   uint32_t rb[R];        // read bases (kNeverBase for rows past the read)
   float miss[R];         // mismatch factor of rows 1 .. R-1 (the same for both halves)
+  float hit[GEN ? R : 1];  // match factor (only where some row has P0 > P1; else 1)
   float2 hit0, miss0;    // row 0's match and mismatch factors times the lane's boost, per half
   float2 K[R], X[R];     // k1 f_i and (x/4) f_i (alpha f_n on the last row), both halves
                          // (row 0's times the lane's boost)
   float2 W[R], s[R];     // om of the next column and s of the column finished last
 };
 
-template <int R>
-__device__ __forceinline__ void column_long(LongRows<R>& w, uint32_t hbx, uint32_t hby, float2 s_top, float2 u_top,
+template <int R, bool GEN>
+__device__ __forceinline__ void column_long(LongRows<R, GEN>& w, uint32_t hbx, uint32_t hby, float2 s_top, float2 u_top,
                                             float2 k2, float2 x, float2& u_bot) {
   float2 s_above = s_top;
   float2 nu = u_top;
@@ -84,6 +85,9 @@ __device__ __forceinline__ void column_long(LongRows<R>& w, uint32_t hbx, uint32
       const float fx = w.rb[0] == hbx ? w.hit0.x : w.miss0.x;
       const float fy = w.rb[0] == hby ? w.hit0.y : w.miss0.y;
       mu_new = __fmul2_rn(s_above, make_float2(fx, fy));
+    } else if (GEN) {
+      mu_new = __fmul2_rn(s_above, make_float2(w.rb[r] == hbx ? w.hit[r] : w.miss[r],
+                                               w.rb[r] == hby ? w.hit[r] : w.miss[r]));
     } else {
       mu_new = s_above;
       mul_if_ne(mu_new.x, w.rb[r], hbx, w.miss[r]);
@@ -161,13 +165,16 @@ __device__ __forceinline__ float scale2(float v, int k) {
 // int2) are the warp's shared memory: the boundary read, the boundary written
 // and lane 31's exponents of its four groups of 8 columns.  Returns
 // false when a wait gave up.
-template <int R, int SPAN>
+// ALONE: the drift tier (pairhmm_drift.cu).  The warp runs the strips of its pair
+// one after another, alternating between its two buffers, so nothing is waited for or
+// published; `failed` carries the halves that left the range from strip to strip.
+template <int R, int SPAN, bool GEN = false, bool ALONE = false>
 __device__ __forceinline__ bool long_task(const BatchView& bv, const QueueView& qv, const WorkItem& w, const int g,
                                           const int strip, const int nstrips, const long long task,
                                           const Tables<float>* __restrict__ tb, const Scalars<float>& sc,
                                           const int lane, float4* const bufs, const long long half, const int mine,
                                           float4* __restrict__ ring, float4* __restrict__ oring,
-                                          int2* __restrict__ oexp) {
+                                          int2* __restrict__ oexp, unsigned& failed) {
   constexpr unsigned FULL = 0xffffffffu;
   constexpr double kLn2 = 0.6931471805599453094;
   constexpr int SR = kWarp * R;
@@ -183,7 +190,7 @@ __device__ __forceinline__ bool long_task(const BatchView& bv, const QueueView& 
   const uint8_t* __restrict__ hp2 = bv.hap_bases + ho2 - 1;
   const int M = max(m1, m2);
   const bool first = strip == 0, last = strip == nstrips - 1;
-  if (sc.x < kLongMinExt) {  // the whole pair to the next tiers
+  if (!ALONE && sc.x < kLongMinExt) {  // the whole pair to the next tiers
     if (last && lane < (two ? 2 : 1)) {
       const int64_t o = w.out_begin + g + lane;
       bv.out[o] = __longlong_as_double(0x7ff8000000000000LL);
@@ -205,7 +212,7 @@ __device__ __forceinline__ bool long_task(const BatchView& bv, const QueueView& 
   int* const err = qv.error_flag;
   bool ok = true;
 
-  LongRows<R> rw;
+  LongRows<R, GEN> rw;
   const int i0 = strip * SR;
 #pragma unroll
   for (int r = 0; r < R; ++r) {
@@ -214,12 +221,14 @@ __device__ __forceinline__ bool long_task(const BatchView& bv, const QueueView& 
       const unsigned q = rqual[i];
       rw.rb[r] = rbase[i];
       rw.miss[r] = tb->miss[q];
+      if (GEN) rw.hit[r] = tb->hit[q];
       const float K = tb->K[q], X = (i == n - 1) ? tb->A[q] : tb->X[q];
       rw.K[r] = make_float2(K, K);
       rw.X[r] = make_float2(X, X);
     } else {  // past the read: pass u down the column
       rw.rb[r] = kNeverBase;
       rw.miss[r] = 0.f;
+      if (GEN) rw.hit[r] = 0.f;
       rw.K[r] = make_float2(0.f, 0.f);
       rw.X[r] = make_float2(1.f, 1.f);
     }
@@ -262,8 +271,12 @@ __device__ __forceinline__ bool long_task(const BatchView& bv, const QueueView& 
   float4 nxt = make_float4(0.f, 0.f, 0.f, 0.f);
   int2 nexp = make_int2(0, 0);
   int published = 0;  // blocks of the strip above known to be published
+  if (ALONE && !first) {
+    src = bufs + (long long)(mine ^ 1) * half;
+    src_exp = reinterpret_cast<const int2*>(src + qv.long_exp_off);
+  }
   auto load_window = [&](int wn) {
-    if (published < min(wn + 2, nwin)) {
+    if (!ALONE && published < min(wn + 2, nwin)) {
       const unsigned long long v = wait_task(above, min(wn + 2, nwin), err, ok);
       published = task_blocks(v);
       if (src == nullptr) {
@@ -299,7 +312,6 @@ __device__ __forceinline__ bool long_task(const BatchView& bv, const QueueView& 
   int bmx = kLongNone, bmy = kLongNone;     // exponents of the bottom row's maxima (this lane's columns)
   const bool lane0 = lane == 0;
 
-  int in_x = kLongNone, in_y = kLongNone;  // exponents of the window's largest inputs
   auto add_total = [&](double& acc, int e, double& tot, int& E) {
     if (acc > 0.0) {
       if (E == kLongNone) {
@@ -317,6 +329,7 @@ __device__ __forceinline__ bool long_task(const BatchView& bv, const QueueView& 
     acc = 0.0;
   };
 
+  int in_x = kLongNone, in_y = kLongNone;  // exponents of the window's largest inputs
   // new exponents for the steps from t on, from the state, the lanes above and
   // the staged inputs; `stage`: a window starts, its inputs go into the ring.
   // INNER: no lane comes to a haplotype's end in these steps.
@@ -430,7 +443,7 @@ __device__ __forceinline__ bool long_task(const BatchView& bv, const QueueView& 
     // inputs come in the scale of the lane above: fold the difference into row 0
     const int upx = __shfl_up_sync(FULL, ex, 1) - ex, upy = __shfl_up_sync(FULL, ey, 1) - ey;  // (lane 0: 0)
     const float2 in = make_float2(pow2T(max(-127, min(126, upx)), 0.f), pow2T(max(-127, min(126, upy)), 0.f));
-    rw.hit0 = in;
+    rw.hit0 = GEN ? make_float2(rw.hit[0] * in.x, rw.hit[0] * in.y) : in;
     rw.miss0 = make_float2(rw.miss[0] * in.x, rw.miss[0] * in.y);
     rw.K[0] = make_float2(K0 * in.x, K0 * in.y);
     rw.X[0] = make_float2(X0 * in.x, X0 * in.y);
@@ -458,7 +471,7 @@ __device__ __forceinline__ bool long_task(const BatchView& bv, const QueueView& 
     float2 s_in = shfl_up2(rw.s[R - 1]);
     u_in = lane0 ? make_float2(rec.y, rec.w) : u_in;
     s_in = lane0 ? make_float2(rec.x, rec.z) : s_in;
-    column_long<R>(rw, hbx, hby, s_top, u_in, k2, x, u_bot);
+    column_long(rw, hbx, hby, s_top, u_in, k2, x, u_bot);
     s_top = s_in;
     if (STEADY) {
       acc32 = __fadd2_rn(acc32, u_bot);
@@ -515,7 +528,7 @@ __device__ __forceinline__ bool long_task(const BatchView& bv, const QueueView& 
     flush_acc();
     // the block laid down at the end of the last window: its stores have long
     // arrived, so the release costs no wait
-    if (q == 0 && !last && lane0 && wn > 0) st_release(word, tag | (unsigned)wn);
+    if (!ALONE && q == 0 && !last && lane0 && wn > 0) st_release(word, tag | (unsigned)wn);
     if (q == 1 && !first && wn + 1 < nwin) load_window(wn + 1);
   };
   for (int wn = 0; wn < nwin; ++wn) {
@@ -549,22 +562,23 @@ __device__ __forceinline__ bool long_task(const BatchView& bv, const QueueView& 
   }
 
   // the halves that left what this tier keeps: their decay so far is over the rate
-  unsigned failed = 0;
-  if (!first) {
+  unsigned lost = ALONE ? failed : 0u;
+  if (!ALONE && !first) {
     const unsigned long long v = wait_task(above, nwin, err, ok);
     if (!ok) return false;
-    failed = task_fail(v);
+    lost = task_fail(v);
   }
-  const int cap = long_max_bits(min(n, i0 + SR));
+  const int cap = ALONE && nstrips == 1 ? INT_MAX : long_max_bits(min(n, i0 + SR));
   if (!last) {
     bmx = __reduce_max_sync(FULL, bmx);
     bmy = __reduce_max_sync(FULL, bmy);
-    if (bmx < -cap) failed |= 1u;
-    if (bmy < -cap) failed |= 2u;
+    if (bmx < -cap) lost |= 1u;
+    if (bmy < -cap) lost |= 2u;
+    if (ALONE) failed = lost;
     __syncwarp();
-    if (lane0) {
+    if (!ALONE && lane0) {
       __threadfence();
-      st_release(word, tag | ((unsigned long long)failed << 30) | (unsigned)nwin);
+      st_release(word, tag | ((unsigned long long)lost << 30) | (unsigned)nwin);
     }
   } else {
     double lnN = 0.0;
@@ -583,12 +597,12 @@ __device__ __forceinline__ bool long_task(const BatchView& bv, const QueueView& 
           spill_pair<float>(qv, w.read, h, o);
         }
       };
-      write(totx, Ex, (failed & 1u) != 0, m1, h1, w.out_begin + g);
-      if (two) write(toty, Ey, (failed & 2u) != 0, m2, h2, w.out_begin + g + 1);
+      write(totx, Ex, (lost & 1u) != 0, m1, h1, w.out_begin + g);
+      if (two) write(toty, Ey, (lost & 2u) != 0, m2, h2, w.out_begin + g + 1);
     }
-    if (lane0) st_release(word, (unsigned)nwin);
+    if (!ALONE && lane0) st_release(word, (unsigned)nwin);
   }
-  if (qv.strip_runs != nullptr && lane0) {
+  if (!ALONE && qv.strip_runs != nullptr && lane0) {
     atomicAdd(qv.strip_runs, 1ull);
     atomicAdd(qv.strip_runs + 1, 1ull);
   }
@@ -643,6 +657,7 @@ pairhmm_long_kernel(const __grid_constant__ BatchView bv, const __grid_constant_
     const int j = (int)((long long)k - qv.long_off[lo]);
     const int g = 2 * (j / nstrips), strip = j % nstrips;
     bool ok = true;
+    unsigned failed = 0;
     if (strip < nstrips - 1) {
       if (reader[turn] >= 0) wait_task(qv.long_words + reader[turn], reader_blocks[turn], qv.error_flag, ok);
       const int64_t h = w.hap_begin + g;
@@ -657,7 +672,7 @@ pairhmm_long_kernel(const __grid_constant__ BatchView bv, const __grid_constant_
   case r:                                                                                                        \
     if constexpr (r >= LO && r <= HI)                                                                            \
       ok = long_task<r, SPAN>(bv, qv, w, g, strip, nstrips, (long long)k, &tab, sc, lane, bufs, half, 2 * gw + turn,  \
-                        rings[wid][0], rings[wid][1], exps[wid]);                                                        \
+                        rings[wid][0], rings[wid][1], exps[wid], failed);                                                \
     break;
         VD_LCASE(4) VD_LCASE(5) VD_LCASE(6) VD_LCASE(7) VD_LCASE(8)
 #undef VD_LCASE
