@@ -96,7 +96,7 @@ constexpr int kUnroll = 8;
 // Reads of several strips, and pairs of the drift tier, need a gap-continuation
 // probability of at least this for FP32 to hold them (pairhmm_long.cuh); below
 // it they go to FP64.
-constexpr float kLongMinExt = 0.0025f;
+constexpr float kLongMinExt = 0.01f;
 
 // Row layout of one read (lane L, register r of strip s holds row
 // i = s*32R + L*R + r - v, 0-based):

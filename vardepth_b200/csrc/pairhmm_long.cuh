@@ -104,16 +104,18 @@ __device__ __forceinline__ void column_long(LongRows<R, GEN>& w, uint32_t hbx, u
   u_bot = nu;
 }
 
-// Steps between two choices of the lanes' exponents.  A lane's bound counts
-// the lanes that a path can come down from by matches alone (span / R + 1)
-// at their full value, so a path that runs down a column by insertions
-// instead lies up to (span + 2 R) log2(4/x) bits and a gap opening below it: at
-// x = 0.1 190 bits for 16 steps, of the 226 between the bound and 2^-126;
-// smaller x needs 8.  Below kLongMinExt (pairhmm_kernel.cuh) a read that hangs
-// off the haplotype's end has no cheap way down, its best path lies hundreds of
-// bits below one that ends there, and the pair goes to the FP64 tier (restated
-// on the CPU against the oracle over reads hanging off by up to 40 bases: exact
-// to FP32 rounding from x = 0.003 up, off by up to 1e-1 log10 at 0.001).
+// Steps between two choices of the lanes' exponents.  A lane's bound takes every
+// match at its full value, so in a path that inserts instead the lane's last cells lie
+// up to (span + 2 R) log2(4/x) bits and a gap opening below it: at x = 0.1 185 bits for
+// 16 steps of 8 rows, of the 226 between the bound and 2^-126, at 0.08 196; smaller x
+// needs 8 steps (200 bits at 0.02).  Below kLongMinExt (pairhmm_kernel.cuh) the pair
+// goes to the FP64 tier.  Measured against the long double oracle on 2,688 pairs of
+// reads that hang off their haplotype by 20 bases to three quarters of their length,
+// where every placement of the inserted run weighs the same: within 1e-5 log10 from
+// x = 0.007 up, off by 6e-5 at 0.005 and 4e-2 at 0.003.  (With a bound that let a path
+// come down by span / R + 1 lanes of matches after any number of insertions, and with
+// the inputs of the whole window in it, up to 0.3 at 0.1 and 1 at 0.08; the closer bound
+// costs 4% on error-rich 1-10 kb reads.)
 constexpr int kLongSpan = 16, kLongSpanShort = 8;
 
 __device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long* p) {
@@ -237,31 +239,32 @@ __device__ __forceinline__ bool long_task(const BatchView& bv, const QueueView& 
   }
   const float K0 = rw.K[0].x, X0 = rw.X[0].x;  // row 0's own factors (those in rw carry the lane factor)
   // bits a path loses when it crosses this lane by insertions, one run of them
-  // (X per row) or single ones (K), summed over the lanes down to this one (the lanes past the read lose nothing, and no path
-  // to a lane of the read crosses its last one)
+  // (X per row) or single ones (K), summed over the lanes down to this one (the
+  // lanes past the read lose nothing, and no path to a lane of the read crosses its
+  // last one)
   const int used = (min(SR, n - i0) + R - 1) / R;  // lanes holding read rows
-  constexpr int reach = SPAN / R + 1;
-  int cross = 0, slack = 0, row_bits = 30;
+  constexpr int near = (SPAN + R) / (R + 1);       // lanes a path can come down by matches alone (rescale)
+  int cross = 0, far_off = 0, row_min = 30, row_max = 0;
   {
-    float b = 0.f;
+    float b = 0.f, top = 0.f;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       const float c = -log2f(fmaxf(rw.X[r].x, rw.K[r].x));
       b += c;
-      if (i0 + lane * R + r < n) row_bits = min(row_bits, (int)floorf(fminf(30.f, c - 0.01f)));
+      top = fmaxf(top, fminf(96.f, c));
+      if (i0 + lane * R + r < n) row_min = min(row_min, (int)floorf(fminf(30.f, c - 0.01f)));
     }
-    row_bits = max(0, __reduce_min_sync(FULL, row_bits));  // per row, at least
+    row_min = max(0, __reduce_min_sync(FULL, row_min));  // bits per row, at least
+    row_max = __reduce_max_sync(FULL, lane < used - 1 ? (int)ceilf(top + 0.01f) : 0);  // and at most
     // (at most 96, so that neighbours' exponents differ by less than a float's range)
-    const int bits = max(0, (int)floorf(fminf(96.f, b - 0.01f)));
-    // a path may take its matches in whichever lanes cost most by insertions
-    slack = reach * max(0, __reduce_max_sync(FULL, lane < used - 1 ? bits : 0) -
-                               __reduce_min_sync(FULL, lane < used - 1 ? bits : 1 << 20));
-    cross = lane < used - 1 ? bits : 0;
+    const int own = lane < used - 1 ? max(0, (int)floorf(fminf(96.f, b - 0.01f))) : 0;
+    cross = own;
 #pragma unroll
     for (int o = 1; o < kWarp; o <<= 1) {
       const int v = __shfl_up_sync(FULL, cross, o);
       if (lane >= o) cross += v;
     }
+    far_off = row_max * (SPAN - lane) - (cross - own);
   }
 
   // boundary above: lane i of window w holds column 32 w + i, raw, with the
@@ -329,9 +332,11 @@ __device__ __forceinline__ bool long_task(const BatchView& bv, const QueueView& 
     acc = 0.0;
   };
 
-  int in_x = kLongNone, in_y = kLongNone;  // exponents of the window's largest inputs
   // new exponents for the steps from t on, from the state, the lanes above and
-  // the staged inputs; `stage`: a window starts, its inputs go into the ring.
+  // the inputs of these steps; `stage`: a window starts, its inputs go into the ring.
+  // (Inputs of later steps do not count: along a run of insertions the boundary
+  // rises by log2(4/x) bits a column, and every column of it carries as much of the
+  // final sum.  They may leave the range in the ring, which is filled again then.)
   // INNER: no lane comes to a haplotype's end in these steps.
   auto rescale = [&](auto inner_tag, const int t, const bool stage) {
     constexpr bool INNER = decltype(inner_tag)::value;
@@ -349,43 +354,54 @@ __device__ __forceinline__ bool long_task(const BatchView& bv, const QueueView& 
       mx = fmaxf(mx, fmaxf(rw.s[r].x, rw.W[r].x));
       my = fmaxf(my, fmaxf(rw.s[r].y, rw.W[r].y));
     }
-    if (stage) {
-      // records past a haplotype's end do not count (nor do they lead anywhere)
-      const int p = t + lane;
-      in_x = __reduce_max_sync(FULL, INNER || p <= m1 ? state_exponent(fmaxf(nxt.x, nxt.y)) + nexp.x : kLongNone);
-      in_y = __reduce_max_sync(FULL, INNER || p <= m2 ? state_exponent(fmaxf(nxt.z, nxt.w)) + nexp.y : kLongNone);
-    }
+    // records past a haplotype's end do not count (nor do they lead anywhere)
+    const int p = (t & ~(kWarp - 1)) + lane;
+    const bool soon = (unsigned)(p - t) < (unsigned)SPAN;
+    const int in_x = __reduce_max_sync(FULL, soon && (INNER || p <= m1) ? state_exponent(fmaxf(nxt.x, nxt.y)) + nexp.x : kLongNone);
+    const int in_y = __reduce_max_sync(FULL, soon && (INNER || p <= m2) ? state_exponent(fmaxf(nxt.z, nxt.w)) + nexp.y : kLongNone);
     const int ox = state_exponent(mx), oy = state_exponent(my);
-    // largest exponent the lane can reach in the coming steps.  A lane that
-    // has gone past the haplotype's last column feeds nothing any more.
+    // Largest exponent the lane can reach in the coming steps, from its own state,
+    // the lanes above and the inputs (a lane above lane 0).  A path that comes down d
+    // lanes takes a step for each, and one for each row it takes by a match (what
+    // lies on the diagonal into the lane below is a match ahead): of the (d-1) R + 1
+    // rows to the lane's first, at most SPAN - d + 1 are matches, which may lose
+    // nothing, and the others cost insertions.  That leaves the lanes d <= near at
+    // their full value, and the others less the bits of the lanes crossed, row_max
+    // back for each match.  Near the haplotype's end the columns left bound the
+    // matches too.  A lane that has gone past the last column feeds nothing any more.
+    // (A shuffle from above lane 0 returns the lane's own value.)
     auto bound = [&](int o, int e, int in, int mh) -> int {
       int v = o + e;  // (far below every real one when there is nothing)
       if (!INNER && t - 1 - lane > mh) v = kLongNone;
-      if (lane0 && (INNER || t <= mh)) v = max(v, in);
-      // far: the best of the lanes above less the bits lost on the way; h: the
-      // best of the lanes within reach by matches alone.  Near the haplotype's
-      // end fewer columns are left for matches: the other rows cost insertions.
-      // (A shuffle from above lane 0 returns the lane's own value.)
-      int far = v + cross, h = v;
-      if (!INNER) {
-        const int cols = min(SPAN, mh - (t - 1 - lane));
-        far -= row_bits * (SPAN - cols);
-#pragma unroll
-        for (int d = 1; d <= reach; ++d)
-          h = max(h, __shfl_up_sync(FULL, v - row_bits * max(0, R * (d - 1) + 1 - cols), d));
-      } else {
-        int left = reach;
+      if (!INNER && t > mh) in = kLongNone;
+      const int cols = INNER ? SPAN : max(0, min(SPAN, mh - (t - 1 - lane)));  // columns left
+      int h = v;
+      if (INNER) {
+        int left = near;
 #pragma unroll
         for (int o2 = 1; o2 < kWarp; o2 <<= 1) {
           if (left > 0) h = max(h, __shfl_up_sync(FULL, h, min(o2, left)));
           left -= min(o2, left);
         }
-      }
+      } else {
 #pragma unroll
-      for (int o2 = 1; o2 < kWarp; o2 <<= 1) far = max(far, __shfl_up_sync(FULL, far, o2));
-      far -= cross;
-      const int q = __shfl_up_sync(FULL, far, reach) + slack;
-      if (lane >= reach) h = max(h, q);
+        for (int d = 1; d <= near; ++d)
+          h = max(h, __shfl_up_sync(FULL, v - row_min * max(0, R * (d - 1) + 1 - min(SPAN - d + 1, cols + 1)), d));
+      }
+      if (lane < near) h = max(h, in);
+      int a = v + cross + row_max * lane;
+#pragma unroll
+      for (int o2 = 1; o2 < kWarp; o2 <<= 1) a = max(a, __shfl_up_sync(FULL, a, o2));
+      a = __shfl_up_sync(FULL, a, near + 1);
+      a = max(lane > near ? a : kLongNone, in - row_max) + far_off;
+      if (!INNER) {
+        int b = v + cross + row_max * cols;
+#pragma unroll
+        for (int o2 = 1; o2 < kWarp; o2 <<= 1) b = max(b, __shfl_up_sync(FULL, b, o2));
+        b = __shfl_up_sync(FULL, b, near + 1);
+        a = min(a, max(lane > near ? b : kLongNone, in + row_max * SPAN) + far_off - row_max * (SPAN - lane));
+      }
+      if (lane >= near) h = max(h, a);
       if (used < kWarp) {
         // the lanes past the read pass u down the column unchanged
         const int pad = __reduce_max_sync(FULL, lane >= used ? v : kLongNone);
@@ -428,15 +444,9 @@ __device__ __forceinline__ bool long_task(const BatchView& bv, const QueueView& 
     // the window's inputs in lane 0's scale
     const int e0x = __shfl_sync(FULL, nx, 0), e0y = __shfl_sync(FULL, ny, 0);
     __syncwarp();
-    if (stage) {
+    if (stage || __shfl_sync(FULL, ex, 0) != e0x || __shfl_sync(FULL, ey, 0) != e0y) {
       const int sx = nexp.x - e0x, sy = nexp.y - e0y;
       ring[lane] = make_float4(scale2(nxt.x, sx), scale2(nxt.y, sx), scale2(nxt.z, sy), scale2(nxt.w, sy));
-    } else {
-      const int sx = __shfl_sync(FULL, ex, 0) - e0x, sy = __shfl_sync(FULL, ey, 0) - e0y;
-      if (sx != 0 || sy != 0) {
-        const float4 raw = ring[lane];
-        ring[lane] = make_float4(scale2(raw.x, sx), scale2(raw.y, sx), scale2(raw.z, sy), scale2(raw.w, sy));
-      }
     }
     ex = nx;
     ey = ny;
@@ -508,9 +518,12 @@ __device__ __forceinline__ bool long_task(const BatchView& bv, const QueueView& 
   };
   auto group = [&](auto steady_tag, const int wn, const int q) {
     const int t = wn * kWarp + q * 8;
+    // (the last choice of exponents in the window was the last use of its records)
+    constexpr int kLoadAt = (kWarp - SPAN) / 8;
     if constexpr (decltype(steady_tag)::value) {
       if (fetched != t) fetch(t);
       if (((q * 8) & (SPAN - 1)) == 0) rescale(steady_tag, t, q == 0);
+      if (q == kLoadAt && !first && wn + 1 < nwin) load_window(wn + 1);
       const int sx = ((int)reinterpret_cast<uintptr_t>(hp1) + t - lane) & 3, sy = ((int)reinterpret_cast<uintptr_t>(hp2) + t - lane) & 3;
       const uint32_t xa = __funnelshift_r(px0, px1, sx * 8), xb = __funnelshift_r(px1, px2, sx * 8);
       const uint32_t ya = __funnelshift_r(py0, py1, sy * 8), yb = __funnelshift_r(py1, py2, sy * 8);
@@ -522,6 +535,7 @@ __device__ __forceinline__ bool long_task(const BatchView& bv, const QueueView& 
              __byte_perm(u < 4 ? ya : yb, 0, 0x4440 + (u & 3)));
     } else {
       if (((q * 8) & (SPAN - 1)) == 0) rescale(steady_tag, t, q == 0);
+      if (q == kLoadAt && !first && wn + 1 < nwin) load_window(wn + 1);
 #pragma unroll 1
       for (int u = 0; u < 8; ++u) step(steady_tag, t + u, 0u, 0u);
     }
@@ -529,7 +543,6 @@ __device__ __forceinline__ bool long_task(const BatchView& bv, const QueueView& 
     // the block laid down at the end of the last window: its stores have long
     // arrived, so the release costs no wait
     if (!ALONE && q == 0 && !last && lane0 && wn > 0) st_release(word, tag | (unsigned)wn);
-    if (q == 1 && !first && wn + 1 < nwin) load_window(wn + 1);
   };
   for (int wn = 0; wn < nwin; ++wn) {
     // columns of this window: 32 wn - 31 .. 32 wn + 31
