@@ -151,6 +151,12 @@ __device__ __forceinline__ void process_item(const BatchView& bv, const QueueVie
   bool fail = false;  // a strip boundary left the range
 
   const long long half = qv.scratch_stride;
+  // A cell that FP32 loses at a boundary lies 2^-246 below that row's largest, and the
+  // path through it may still win later if the others lose as much.  A read of
+  // several strips is therefore kept under the rule of one strip: its likelihood at
+  // most 200 bits below a perfect match's, counted over all its strips.
+  constexpr bool kRow0Floor = sizeof(T) == 4;
+  constexpr int kMaxDecay = 200;
 
   // One strip of rows.
   // FIRST and LAST are compile-time tags, so the steady loop carries no
@@ -208,7 +214,9 @@ __device__ __forceinline__ void process_item(const BatchView& bv, const QueueVie
       // than 1e-300 below that row maximum
       const double Zc = ANCH ? fmax(Zs, 1e-300 * (double)rmax) : Zs;
       const double lnC0 = sc.ln_c + (ANCH ? 0.0 : log((double)(m + 1)));
-      const bool ok = !fail && Zs >= (double)sc.final_floor && Zs < HUGE_VAL;
+      // (FP32 strips: the floor holds from row 0 on, whatever the renormalisations)
+      const double floor = kRow0Floor && E > 0 ? ldexp((double)sc.final_floor, E) : (double)sc.final_floor;
+      const bool ok = !fail && Zs >= floor && Zs < HUGE_VAL;
       if (ok || qv.spill == nullptr) {
         bv.out[o] = (Zc > 0.0 ? log(Zc) : -HUGE_VAL) - lnC0 + lnN - (double)E * kLn2;
       } else {
@@ -401,6 +409,7 @@ __device__ __forceinline__ void process_item(const BatchView& bv, const QueueVie
       }
       __syncwarp();
       E += ks;
+      if (kRow0Floor && E > kMaxDecay) return false;
     }
     return true;
   };
