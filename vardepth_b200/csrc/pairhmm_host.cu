@@ -947,10 +947,18 @@ struct Layout {
   int64_t long_stride;     // the same of the long-read kernel (two boundary buffers)
   int64_t drift_stride;    // the same of the drift tier (0: reads of one strip only)
   int drift_blocks;        // blocks of the drift tier the scratch holds
+  bool apart;              // the long-read kernel's buffers have bytes of their own
 };
 
-Layout layout_for(const vd_engine* e, const HostChunk& c) {
-  const int64_t warps = max_grid_warps(e), warps_long = long_warps(e, c);
+// Warps of the tiers that keep strip boundaries: all of them when reads take several
+// strips, else the robust tier's alone.
+int64_t strip_warps(const vd_engine* e, bool any_strip) {
+  const int64_t warps = max_grid_warps(e);
+  return any_strip ? warps : std::min<int64_t>(warps, (int64_t)kRobustBlocks * kWarpsPerBlock);
+}
+
+Layout layout_for(const vd_engine* e, const HostChunk& c, size_t budget = SIZE_MAX) {
+  const int64_t warps = strip_warps(e, c.any_strip), warps_long = long_warps(e, c);
   Layout L{};
   size_t off = 0;
   auto take = [&](size_t bytes) { size_t o = off; off = align_up(off + std::max<size_t>(bytes, 1), 256); return o; };
@@ -974,20 +982,22 @@ Layout layout_for(const vd_engine* e, const HostChunk& c) {
   L.o_cnt = take(16 * sizeof(unsigned long long));
   // one word per task of the long-read kernel, right behind the counters (cleared with them)
   L.o_lword = take(c.long_off.empty() ? 0 : (size_t)c.long_off.back() * sizeof(unsigned long long));
-  // one boundary per warp slot of the tiers.  The long-read kernels use the same
-  // bytes as two buffers per warp: the rescue tiers start when they are done; only
-  // the single-read kernel beside them, when it strip-mines reads too (long
-  // reads with Phred 0 or 1 bases), needs its own.
+  // one boundary per warp slot of the tiers.  The long-read kernel uses the same
+  // bytes as two buffers per warp: the rescue tiers start when it is done; only the
+  // single-read kernel beside it, when it strip-mines reads too (long reads with
+  // Phred 0 or 1 bases), needs its own, or where the budget does not hold both, waits
+  // for the long-read kernel.
   L.scratch_stride = c.any_long ? (int64_t)c.max_hap + 1 : 0;
   L.long_stride = c.n_long > 0 ? 2 * long_buffer_records(c.max_hap) : 0;
   const int64_t own = std::max<int64_t>(1, L.scratch_stride) * warps, shared = L.long_stride * warps_long;
-  L.o_scratch = take((size_t)(c.strip_singles ? own : std::max(own, shared)) * sizeof(double2));
-  L.o_long = c.strip_singles ? take((size_t)shared * sizeof(double2)) : L.o_scratch;
+  L.apart = c.strip_singles && off + (size_t)(own + shared) * sizeof(double2) + 512 <= budget;
+  L.o_scratch = take((size_t)(L.apart ? own : std::max(own, shared)) * sizeof(double2));
+  L.o_long = L.apart ? take((size_t)shared * sizeof(double2)) : L.o_scratch;
   // the drift tier runs after both and takes as many blocks as the larger holds
   L.drift_stride = c.any_strip ? 2 * long_buffer_records(c.max_hap) : 0;
   L.drift_blocks = e->grid_drift;
   if (c.any_strip)
-    L.drift_blocks = (int)std::min<int64_t>(L.drift_blocks, (c.strip_singles ? own : std::max(own, shared)) /
+    L.drift_blocks = (int)std::min<int64_t>(L.drift_blocks, (L.apart ? own : std::max(own, shared)) /
                                                                 (L.drift_stride * kWarpsPerBlock));
   L.total = off;
   return L;
@@ -1219,6 +1229,7 @@ int enqueue_tiers(vd_plan* pl, int* launches, bool capturing = false, Tiers whic
     q.items = (const WorkItem*)(d + L.o_items) + np + nl;
     q.n_items = (long long)ns;
     if (q.n_items > 0) {
+      if (pl->chunk.strip_singles && !L.apart) VD_CUDA(cudaStreamWaitEvent(pl->stream, pl->side->join[0], 0));
       err = f64 ? launch_f64(anch, bv, q, &dt->f64, ht->s64, 1, e->grid[1][anch], pl->stream)
                 : launch_f32(anch, bv, q, &dt->f32, ht->s32, 0, e->grid[0][anch], pl->stream);
       if (err != cudaSuccess) return cuda_fail(err, "primary tier launch");
@@ -1573,7 +1584,9 @@ int vd_forward(vd_engine* e, const vd_batch* b, const vd_params* p, double* out,
   s.pairs = n_out;
   if ((rc = ensure_tables(e, p))) return rc;
   const bool offsets = p->quality_offsets != nullptr;
-  const int64_t warps = max_grid_warps(e);
+  const bool plain = p->schedule == VD_SCHEDULE_PLAIN;
+  BuildOpts lbo = build_opts(e);
+  lbo.item_limit = batch_item_limit(e, b, p);
 
   // chunk boundaries: regions (region form) or reads (pair form)
   PairGroups pg;
@@ -1582,17 +1595,33 @@ int vd_forward(vd_engine* e, const vd_batch* b, const vd_params* p, double* out,
   const int64_t units = pair_form ? b->n_reads : b->n_regions;
   // bytes per unit, estimated from inputs; a chunk grows until the estimate
   // reaches the budget (accelerator.py:118-121 semantics)
+  int64_t max_read = 0;
+  for (int64_t r = 0; r < b->n_reads; ++r) max_read = std::max<int64_t>(max_read, b->read_off[r + 1] - b->read_off[r]);
+  const bool any_strip = max_read + p->anchored > kStripRows;
+  const bool strip_tasks = !pair_form && lbo.long_warp && p->precision != VD_PRECISION_FLOAT64 && !p->anchored;
   auto unit_bytes = [&](int64_t u) -> int64_t {
+    // (a read of several strips has an item per haplotype, or with strip tasks one per
+    // long_group of them and a word per strip and two haplotypes)
+    auto strip_bytes = [&](int64_t r, int64_t nh) -> int64_t {
+      const int64_t n = b->read_off[r + 1] - b->read_off[r] + p->anchored;
+      if (n <= kStripRows) return 0;
+      const int64_t strips = (n + kWarp * lbo.long_R - 1) / (kWarp * lbo.long_R);
+      if (!strip_tasks) return nh * (int64_t)sizeof(WorkItem);
+      const int64_t items = (nh + lbo.long_group - 1) / lbo.long_group;
+      return items * ((int64_t)sizeof(WorkItem) + 8) + 8 * strips * (nh / 2 + items);
+    };
     if (pair_form) {
       const int64_t n = b->read_off[u + 1] - b->read_off[u];
       const int64_t np = pg.start[u + 1] - pg.start[u];
-      return 2 * n + 64 + np * (4 + 8 + 8 + 32) + 64;
+      return 2 * n + 64 + np * (4 + 8 + 8 + 32) + 64 + (plain ? np * (int64_t)sizeof(WorkItem) : strip_bytes(u, np));
     }
     const int64_t r0 = b->region_read_off[u], r1 = b->region_read_off[u + 1];
     const int64_t h0 = b->region_hap_off[u], h1 = b->region_hap_off[u + 1];
     const int64_t np = (r1 - r0) * (h1 - h0);
+    int64_t extra = plain ? np * (int64_t)sizeof(WorkItem) : 0;
+    if (any_strip) for (int64_t r = r0; r < r1; ++r) extra += strip_bytes(r, h1 - h0);
     return 2 * (b->read_off[r1] - b->read_off[r0]) + (r1 - r0) * 64 + (b->hap_off[h1] - b->hap_off[h0]) +
-           (h1 - h0) * 8 + np * (8 + 32);
+           (h1 - h0) * 16 + np * (8 + 32) + extra;
   };
   // DP cells per unit: large batches are cut into several chunks so that the
   // host work of one chunk overlaps the kernels of the previous one
@@ -1606,8 +1635,6 @@ int vd_forward(vd_engine* e, const vd_batch* b, const vd_params* p, double* out,
   for (int64_t u = 0; u < units; ++u) total_cells += unit_cells(u);
   // warp items of the long-read kernel (reads longer than a strip, up to
   // long_group haplotypes each)
-  BuildOpts lbo = build_opts(e);
-  lbo.item_limit = batch_item_limit(e, b, p);
   int64_t long_items = 0;
   if (lbo.long_warp && p->precision != VD_PRECISION_FLOAT64 && !p->anchored) {
     auto long_reads = [&](int64_t r0, int64_t r1) {
@@ -1635,13 +1662,12 @@ int vd_forward(vd_engine* e, const vd_batch* b, const vd_params* p, double* out,
   const int64_t chunk_cells = n_pipe > 1 ? (total_cells + n_pipe - 1) / n_pipe : INT64_MAX;
 
   int64_t fixed = pair_form ? (b->hap_off[b->n_haps] - b->hap_off[0]) + 8 * b->n_haps : 0;
-  int64_t max_hap = 0, max_read = 0;
+  int64_t max_hap = 0;
   for (int64_t h = 0; h < b->n_haps; ++h) max_hap = std::max<int64_t>(max_hap, b->hap_off[h + 1] - b->hap_off[h]);
-  for (int64_t r = 0; r < b->n_reads; ++r) max_read = std::max<int64_t>(max_read, b->read_off[r + 1] - b->read_off[r]);
-  const int64_t scratch_warps = max_read + p->anchored > kStripRows ? warps : std::min<int64_t>(warps, (int64_t)kRobustBlocks * kWarpsPerBlock);
   // (two boundary buffers per warp of the long-read kernel where it runs)
   const int64_t long_w = (int64_t)e->grid_long[lbo.long_R == kMaxR ? 1 : 0] * kWarpsPerBlock;
-  fixed += std::max((max_hap + 1) * scratch_warps, max_read > kStripRows ? 2 * long_buffer_records(max_hap) * long_w : 0) *
+  fixed += std::max((max_hap + 1) * strip_warps(e, any_strip),
+                    any_strip && strip_tasks ? 2 * long_buffer_records(max_hap) * long_w : 0) *
                (int64_t)sizeof(double2) +
            64 * 1024;
   const int64_t budget = (int64_t)e->budget;
@@ -1749,13 +1775,18 @@ int vd_forward(vd_engine* e, const vd_batch* b, const vd_params* p, double* out,
     pl.ev_end = sl.ev[2];
     pl.side = &sl.side;
     const double th = now_ms();
-    const bool plain = p->schedule == VD_SCHEDULE_PLAIN;
-    const BuildOpts& bo = lbo;
-    if (pair_form) build_pair_chunk(b, pg, u, u_end, e->htab, offsets, p->anchored != 0, pl.chunk, plain, bo);
-    else build_region_chunk(b, u, u_end, e->htab, offsets, p->anchored != 0, p->precision == VD_PRECISION_MIXED,
-                            pl.chunk, plain, bo);
     HostChunk& c = pl.chunk;
-    pl.L = layout_for(e, c);
+    for (;;) {
+      if (pair_form) build_pair_chunk(b, pg, u, u_end, e->htab, offsets, p->anchored != 0, c, plain, lbo);
+      else build_region_chunk(b, u, u_end, e->htab, offsets, p->anchored != 0, p->precision == VD_PRECISION_MIXED, c,
+                              plain, lbo);
+      pl.L = layout_for(e, c, e->budget);
+      if ((int64_t)pl.L.total <= budget || u_end - u <= 1) break;
+      // more items than the estimate counts (where they are cut, and which long reads
+      // hold Phred 0 or 1, shows only here): fewer units
+      u_end = u + (u_end - u) / 2;
+      c = HostChunk();
+    }
     s.host_ms += now_ms() - th;
     if ((rc = sl.arena.reserve(pl.L.total))) return rc;
     pl.base = (char*)sl.arena.p;
