@@ -177,8 +177,6 @@ struct SideStreams {
   cudaStream_t s[2] = {nullptr, nullptr};
   cudaEvent_t fork = nullptr, join[2] = {nullptr, nullptr};
   cudaError_t create() {
-    if (join[1]) return cudaSuccess;
-    destroy();
     cudaError_t err = cudaEventCreateWithFlags(&fork, cudaEventDisableTiming);
     for (int k = 0; k < 2 && err == cudaSuccess; ++k)
       if ((err = cudaStreamCreateWithPriority(&s[k], cudaStreamNonBlocking, kOwnPriority + (k ? 1 : -1))) ==
@@ -239,23 +237,18 @@ struct vd_engine {
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
     unsigned long long* hcnt = nullptr;  // pinned copy of the tier counters
     char* staging = nullptr;             // pinned, kStagingBytes: the inputs of a small chunk
-    bool ready = false;
-    // the slot's streams, events and pinned memory, made when it is first used
-    // (the second slot only by batches of several chunks)
+    // the slot's streams, events and pinned memory
     cudaError_t create() {
-      if (ready) return cudaSuccess;
-      cudaError_t err = cudaSuccess;
-      if (!stream) err = cudaStreamCreateWithPriority(&stream, cudaStreamNonBlocking, kOwnPriority);
-      for (int k = 0; k < 3 && err == cudaSuccess; ++k)
-        if (!ev[k]) err = cudaEventCreate(&ev[k]);
+      cudaError_t err = cudaStreamCreateWithPriority(&stream, cudaStreamNonBlocking, kOwnPriority);
+      for (int k = 0; k < 3 && err == cudaSuccess; ++k) err = cudaEventCreate(&ev[k]);
       if (err == cudaSuccess) err = side.create();
-      if (err == cudaSuccess && !hcnt) {
+      if (err == cudaSuccess) {
         void* p = nullptr;
-        err = cudaMallocHost(&p, 256 + kStagingBytes);
-        hcnt = (unsigned long long*)p;
-        staging = (char*)p + 256;
+        if ((err = cudaMallocHost(&p, 256 + kStagingBytes)) == cudaSuccess) {
+          hcnt = (unsigned long long*)p;
+          staging = (char*)p + 256;
+        }
       }
-      ready = err == cudaSuccess;
       return err;
     }
     std::vector<double> stage;           // pair-form outputs before the scatter
@@ -1462,9 +1455,14 @@ int vd_engine_create(int device, int64_t memory_mb, vd_engine** out) {
   if ((err = cudaStreamCreateWithPriority(&e->stream, cudaStreamNonBlocking, kOwnPriority)) != cudaSuccess ||
       (err = cudaEventCreate(&e->ev_begin)) != cudaSuccess || (err = cudaEventCreate(&e->ev_mid)) != cudaSuccess ||
       (err = cudaEventCreate(&e->ev_end)) != cudaSuccess ||
-      (err = cudaMallocHost((void**)&e->htab, sizeof(TableSet))) != cudaSuccess) {
+      (err = cudaMallocHost((void**)&e->htab, sizeof(TableSet))) != cudaSuccess ||
+      (err = e->side.create()) != cudaSuccess) {
     rc = cuda_fail(err, "engine setup");
   }
+  // (here and not in the first call: a caller that makes an engine per worker and scores
+  // a few regions would pay for it there)
+  for (int k = 0; k < 2 && !rc; ++k)
+    if ((err = e->slots[k].create()) != cudaSuccess) rc = cuda_fail(err, "engine pipeline setup");
   if (!rc) rc = init_engine_grids(e);
   if (rc) { vd_engine_destroy(e); return rc; }
   *out = e;
@@ -1763,7 +1761,6 @@ int vd_forward(vd_engine* e, const vd_batch* b, const vd_params* p, double* out,
     if (bytes > budget) return fail(VD_ENOMEM, "One pair exceeds CUDA workspace budget");
     vd_engine::Slot& sl = e->slots[chunk_index & 1];
     if ((rc = finish(sl))) return rc;  // the slot's previous chunk
-    VD_CUDA(sl.create());
     if (!sl.pl) sl.pl = new vd_plan();
     vd_plan& pl = *sl.pl;
     pl.chunk = HostChunk();
@@ -1827,7 +1824,6 @@ namespace {
 int enqueue_whole(vd_engine* e, const vd_batch* b, const vd_params* p, vd_engine::Slot& sl, vd_stats* s) {
   int rc = ensure_tables(e, p);
   if (rc) return rc;
-  VD_CUDA(sl.create());
   if (!sl.pl) sl.pl = new vd_plan();
   vd_plan& pl = *sl.pl;
   pl.chunk = HostChunk();
@@ -1872,7 +1868,6 @@ int vd_plan_create(vd_engine* e, const vd_batch* b, const vd_params* p, vd_plan*
   std::lock_guard<std::mutex> lk(e->mu);
   DeviceGuard guard(e->device);
   if ((rc = ensure_tables(e, p))) return rc;
-  VD_CUDA(e->side.create());
   vd_plan* pl = new vd_plan();
   pl->eng = e;
   pl->params = *p;
@@ -2142,7 +2137,6 @@ int vd_forward_backward(vd_engine* e, const vd_batch* b, const vd_params* p, int
     gv.count = nullptr;
     const bool aside = n_kernel[0] && n_kernel[1];
     if (aside) {
-      VD_CUDA(e->side.create());
       VD_CUDA(cudaEventRecord(e->side.fork, st_));
       VD_CUDA(cudaStreamWaitEvent(e->side.s[1], e->side.fork, 0));
     }
