@@ -143,7 +143,8 @@ class Interner {
 
   // track_pointers: keep every pointer seen (haplotype objects recur all over
   // a pair list); without it a pointer evicted from the cache counts as a new
-  // object (a read's object recurs only in its own run of pairs)
+  // object (a read's object recurs only in its own run of pairs, or once per
+  // haplotype in a list that goes haplotype by haplotype: full() bounds the objects)
   explicit Interner(bool track_pointers) : track_(track_pointers) {}
 
   // index of the object (b, q, n)
@@ -194,6 +195,14 @@ class Interner {
   }
   int32_t id(int32_t object) const { return objects_[(size_t)object].id; }
 
+  // As many objects as are kept at a time (10 MB): resolve() them, take their ids
+  // and forget() them.
+  bool full() const { return !track_ && objects_.size() >= kObjects; }
+  void forget() {
+    objects_.clear();
+    cache_.assign(kCache, -1);
+  }
+
  private:
   struct Object {
     const unsigned char* b;
@@ -202,7 +211,7 @@ class Interner {
     int32_t id;
     uint64_t h;
   };
-  static constexpr size_t kCache = 4096;
+  static constexpr size_t kCache = 4096, kObjects = (size_t)1 << 18;
   std::vector<int32_t> cache_ = std::vector<int32_t>(kCache, -1);
   bool track_;
   std::vector<Object> objects_;
@@ -228,9 +237,28 @@ int build_plan(const char* const* rs, const unsigned char* const* qs, const int*
   pl.pair_hap.resize((size_t)count);
   // (the objects of the pairs before the first malformed one: an earlier pair that
   // is not DNA is reported before it)
-  int64_t good = 0;
+  int64_t good = 0, read_ids = 0;  // pairs noted; those whose entry is the read's id already
   std::string malformed;
+  std::atomic<bool> dna{true};
+  auto take_read_ids = [&]() {
+    pl.reads.resolve();
+    in_slices(good - read_ids, 32768, [&](int64_t lo, int64_t hi) {
+      bool ok = true;
+      for (int64_t p = read_ids + lo; p < read_ids + hi; ++p) {
+        const int32_t r = pl.reads.id(pl.pair_read[(size_t)p]);
+        pl.pair_read[(size_t)p] = r;
+        ok &= r >= 0;
+      }
+      if (!ok) dna = false;
+    });
+    read_ids = good;
+  };
   for (; good < count; ++good) {
+    if (pl.reads.full()) {
+      take_read_ids();
+      pl.reads.forget();
+      if (!dna) break;
+    }
     const int64_t p = good;
     const int n = rn[p], m = hn[p];
     if (n < 0 || m < 0) {
@@ -244,16 +272,14 @@ int build_plan(const char* const* rs, const unsigned char* const* qs, const int*
     pl.pair_read[(size_t)p] = pl.reads.note((const unsigned char*)rs[p], qs[p], n);
     pl.pair_hap[(size_t)p] = pl.haps.note((const unsigned char*)hs[p], nullptr, m);
   }
-  pl.reads.resolve();
+  take_read_ids();
   pl.haps.resolve();
-  std::atomic<bool> dna{true};
   in_slices(good, 32768, [&](int64_t lo, int64_t hi) {
     bool ok = true;
     for (int64_t p = lo; p < hi; ++p) {
-      const int32_t r = pl.reads.id(pl.pair_read[(size_t)p]), h = pl.haps.id(pl.pair_hap[(size_t)p]);
-      pl.pair_read[(size_t)p] = r;
+      const int32_t h = pl.haps.id(pl.pair_hap[(size_t)p]);
       pl.pair_hap[(size_t)p] = h;
-      ok &= r >= 0 && h >= 0;
+      ok &= h >= 0;
     }
     if (!ok) dna = false;
   });
