@@ -29,10 +29,12 @@ lays out the work list:
 ``autotune`` times candidate settings with resident plans (CUDA events around
 the captured tier graph) on a seeded region sample of the caller's batch,
 coordinate by coordinate, and leaves the best setting on the engine.  Results
-are cached per (device name, sample signature) in a JSON file.
+are cached per device, library, sample signature and gap-continuation class in a
+JSON file: a choice timed with other kernels, or where other tiers run, does not hold.
 """
 from __future__ import annotations
 
+import hashlib
 import json
 import os
 from pathlib import Path
@@ -69,6 +71,19 @@ def signature(read_off, hap_off) -> str:
     hb = np.histogram(m, bins=[0, 257, 1025, 4097, 1 << 30])[0]
     f = lambda h: ",".join(f"{x / max(1, h.sum()):.2f}" for x in h)
     return f"reads[{f(rb)}] haps[{f(hb)}]"
+
+
+def library_revision() -> str:
+    """A short digest of the library's file."""
+    return hashlib.sha256(native.LIB_PATH.read_bytes()).hexdigest()[:16] if native.LIB_PATH.exists() else "none"
+
+
+def cache_key(engine: native.Engine, packed: native.Packed, params) -> str:
+    # long reads choose their exponents twice as often below a gap continuation of 0.08 and run
+    # in FP64 below 0.01
+    ext = "ext<0.01" if params.ext < 0.01 else "ext<0.08" if params.ext < 0.08 else "ext"
+    return (f"{engine.info()['gpu']}|{library_revision()}|{signature(packed.read_off, packed.hap_off)}"
+            f"|anch={params.anchored}|{ext}")
 
 
 def _apply(engine: native.Engine, setting: dict) -> None:
@@ -143,8 +158,7 @@ def autotune(engine: native.Engine, packed: native.Packed, params, repeats: int 
         short_s, long_s = split_samples(packed)
     else:
         short_s, long_s = packed, packed
-    sig_src = packed
-    key = f"{engine.info()['gpu']}|{signature(sig_src.read_off, sig_src.hap_off)}|anch={params.anchored}"
+    key = cache_key(engine, packed, params) if use_cache else None
     cache = {}
     if use_cache and CACHE.exists():
         try:
