@@ -401,9 +401,11 @@ inline int64_t item_work(int64_t stream, int R) { return (stream + kWarp) * (R +
 // largest item was 16 haplotypes of 1,000 columns): kernels 6.5 -> 2.5 ms; 40 in
 // FP64 2.3 -> 1.4, one of 64 reads 0.136 -> 0.104.  Shares of 1/2, 1/4, 1/8 and 1/16
 // ran the 60 regions in 3.7, 2.5, 2.3 and 2.2 ms, but every item costs the host
-// some 45 ns, and the whole call took 7.9, 6.9, 7.1 and 7.3 ms.  It is taken over the whole
+// some 45 ns, and the whole call took 7.9, 6.9, 7.1 and 7.3 ms.  (One FP32 batch; FP64,
+// anchored and packed items go by the same share.)  It is taken over the call's whole
 // batch, so that the items, and the prefixes they share, do not depend on the
-// pipeline's chunks.
+// pipeline's chunks; shards of a batch are batches of their own, whose items may
+// differ, their results not.
 int64_t batch_item_limit(const vd_engine* e, const vd_batch* b, const vd_params* p) {
   auto rows = [&](int64_t r) -> int64_t {
     const int64_t n = b->read_off[r + 1] - b->read_off[r];
@@ -1853,7 +1855,7 @@ int enqueue_whole(vd_engine* e, const vd_batch* b, const vd_params* p, vd_engine
   s->shared_cells = c.shared_cells;
   s->work_items = (int64_t)c.items.size();
   s->batches = 1;
-  s->kernel_launches = launches;
+  s->kernel_launches = launches + (pl.filled ? 1 : 0);  // the -inf fill of the upload
   s->live_bytes = (int64_t)pl.L.total;
   return VD_OK;
 }
@@ -2049,7 +2051,7 @@ int vd_forward_backward(vd_engine* e, const vd_batch* b, const vd_params* p, int
   const bool packed = !f64_only && !store_all && !p->anchored;
   auto kernel_of = [&](int code) { return !packed || code_general(code) ? 2 : code_R(code) >= 5 ? 0 : 1; };
   {
-    // (counting sort over kernel, code and length: the list is in region order)
+    // (a stable sort by kernel, code and length: the list is in region order)
     const size_t n = items.size();
     std::vector<std::pair<uint64_t, uint32_t>> key(n);
     for (size_t k = 0; k < n; ++k) {
