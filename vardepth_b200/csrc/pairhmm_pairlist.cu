@@ -272,14 +272,17 @@ int build_plan(const char* const* rs, const unsigned char* const* qs, const int*
     pl.pair_read[(size_t)p] = pl.reads.note((const unsigned char*)rs[p], qs[p], n);
     pl.pair_hap[(size_t)p] = pl.haps.note((const unsigned char*)hs[p], nullptr, m);
   }
-  take_read_ids();
+  pl.reads.resolve();
   pl.haps.resolve();
   in_slices(good, 32768, [&](int64_t lo, int64_t hi) {
     bool ok = true;
     for (int64_t p = lo; p < hi; ++p) {
+      int32_t r = pl.pair_read[(size_t)p];
+      if (p >= read_ids) r = pl.reads.id(r);
       const int32_t h = pl.haps.id(pl.pair_hap[(size_t)p]);
+      pl.pair_read[(size_t)p] = r;
       pl.pair_hap[(size_t)p] = h;
-      ok &= h >= 0;
+      ok &= r >= 0 && h >= 0;
     }
     if (!ok) dna = false;
   });
