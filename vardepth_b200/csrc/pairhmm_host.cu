@@ -237,18 +237,35 @@ struct vd_engine {
     cudaEvent_t ev[3] = {nullptr, nullptr, nullptr};
     unsigned long long* hcnt = nullptr;  // pinned copy of the tier counters
     char* staging = nullptr;             // pinned, kStagingBytes: the inputs of a small chunk
-    // the slot's streams, events and pinned memory
-    cudaError_t create() {
-      cudaError_t err = cudaStreamCreateWithPriority(&stream, cudaStreamNonBlocking, kOwnPriority);
-      for (int k = 0; k < 3 && err == cudaSuccess; ++k) err = cudaEventCreate(&ev[k]);
-      if (err == cudaSuccess) err = side.create();
-      if (err == cudaSuccess) {
+    bool ready = false, own_streams = false;
+    // the slot's streams, events and pinned memory.  The first slot works on the
+    // engine's own streams: the calls that use either wait for their end.
+    cudaError_t create(cudaStream_t engine_stream = nullptr, const SideStreams* engine_side = nullptr) {
+      if (ready) return cudaSuccess;
+      cudaError_t err = cudaSuccess;
+      if (engine_stream) {
+        stream = engine_stream;
+        side = *engine_side;
+      } else if (!own_streams) {
+        err = cudaStreamCreateWithPriority(&stream, cudaStreamNonBlocking, kOwnPriority);
+        if (err == cudaSuccess) err = side.create();
+        own_streams = err == cudaSuccess;
+        if (!own_streams) {  // (the next call that needs the slot tries again)
+          side.destroy();
+          if (stream) cudaStreamDestroy(stream);
+          stream = nullptr;
+        }
+      }
+      for (int k = 0; k < 3 && err == cudaSuccess; ++k)
+        if (!ev[k]) err = cudaEventCreate(&ev[k]);
+      if (err == cudaSuccess && !hcnt) {
         void* p = nullptr;
         if ((err = cudaMallocHost(&p, 256 + kStagingBytes)) == cudaSuccess) {
           hcnt = (unsigned long long*)p;
           staging = (char*)p + 256;
         }
       }
+      ready = err == cudaSuccess;
       return err;
     }
     std::vector<double> stage;           // pair-form outputs before the scatter
@@ -1462,9 +1479,9 @@ int vd_engine_create(int device, int64_t memory_mb, vd_engine** out) {
     rc = cuda_fail(err, "engine setup");
   }
   // (here and not in the first call: a caller that makes an engine per worker and scores
-  // a few regions would pay for it there)
-  for (int k = 0; k < 2 && !rc; ++k)
-    if ((err = e->slots[k].create()) != cudaSuccess) rc = cuda_fail(err, "engine pipeline setup");
+  // a few regions would pay for it there; the second slot's are made by the first batch
+  // of several chunks)
+  if (!rc && (err = e->slots[0].create(e->stream, &e->side)) != cudaSuccess) rc = cuda_fail(err, "engine pipeline setup");
   if (!rc) rc = init_engine_grids(e);
   if (rc) { vd_engine_destroy(e); return rc; }
   *out = e;
@@ -1494,6 +1511,7 @@ int vd_engine_destroy(vd_engine* e) {
       sl.arena.release();
       for (cudaEvent_t& ev : sl.ev) if (ev) cudaEventDestroy(ev);
       if (sl.hcnt) cudaFreeHost(sl.hcnt);
+      if (!sl.own_streams) continue;
       sl.side.destroy();
       if (sl.stream) cudaStreamDestroy(sl.stream);
     }
@@ -1763,6 +1781,7 @@ int vd_forward(vd_engine* e, const vd_batch* b, const vd_params* p, double* out,
     if (bytes > budget) return fail(VD_ENOMEM, "One pair exceeds CUDA workspace budget");
     vd_engine::Slot& sl = e->slots[chunk_index & 1];
     if ((rc = finish(sl))) return rc;  // the slot's previous chunk
+    VD_CUDA(sl.create());
     if (!sl.pl) sl.pl = new vd_plan();
     vd_plan& pl = *sl.pl;
     pl.chunk = HostChunk();
