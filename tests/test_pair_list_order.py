@@ -45,7 +45,7 @@ def test_the_first_bad_pair_is_reported():
 
 
 PROGRAM = """
-import resource, sys
+import sys
 import numpy as np
 sys.path.insert(0, sys.argv[1])
 from vardepth_b200 import native
@@ -55,12 +55,10 @@ quals = [np.full(8, 30, np.uint8) for _ in reads]
 haps = ["".join(s) for s in rng.choice(list("ACGT"), (100, 20))]
 pl = native.PairList([(s, q, h) for h in haps for s, q in zip(reads, quals)])
 warm = native.pair_list_plan(native.PairList([(reads[0], quals[0], haps[0])]))
-peak = lambda: resource.getrusage(resource.RUSAGE_SELF).ru_maxrss
-for line in open("/proc/self/status"):
-    if line.startswith("VmRSS"):
-        before = int(line.split()[1])
+kb = lambda key: next(int(line.split()[1]) for line in open("/proc/self/status") if line.startswith(key))
+before = kb("VmRSS")
 native.pair_list_plan(pl)
-print((peak() - before) // 1024)
+print((kb("VmHWM") - before) // 1024)  # (ru_maxrss would count what the process it was forked from held)
 """
 
 
