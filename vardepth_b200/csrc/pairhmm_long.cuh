@@ -37,11 +37,11 @@
 // same bits.
 //
 // What bounds it: alone, the chain of a strip's steps; in a full batch, issue
-// slots and latency at 12 warps per SM (115 warp instructions a step for 256 x 2
+// slots and latency at 12 warps per SM (119 warp instructions a step for 256 x 2
 // cells, 72 of them the rows; a quarter of the stalls are boundary words from
 // L2).  Measured against a warp per item (its strips one after another, re-run
 // with measured boosts when they left the FP32 range: 1.11 runs per strip): 30
-// reads of 1-10 kb, 375 pairs, 388 -> 9.2 ms; 400 mixed-length regions 390 -> 28 ms;
+// reads of 1-10 kb, 375 pairs, 388 -> 9.5 ms; 400 mixed-length regions 390 -> 28 ms;
 // 16,000 of them (2.5e12 cells) 804 -> 782 ms, their long reads alone 557 -> 486 ms
 // (2,586 GCUPS).  Exponents every 16 steps cost 12% against every 32, which a
 // 40-base insertion run would defeat; letting a waiting strip fall 1 or 3 blocks
@@ -56,8 +56,10 @@ namespace vd {
 // `rows` rows goes to the drift and FP64 tiers: an error-rich read takes about one
 // bit per row; a random read against a random haplotype takes four to five, and
 // there alignment families that trade places across rows lie hundreds of bits
-// apart (restated on the CPU against the oracle: exact to FP32 rounding below
-// 4.0 bits per row, off by up to 0.2 log10 at 4.0 to 4.4).
+// apart (restated on the CPU with a looser bound of the lanes' exponents than
+// rescale's: exact to FP32 rounding below 4.0 bits per row, off by up to 0.2 log10 at
+// 4.0 to 4.4; with rescale's, 1,344 pairs of hanging reads were within 1.3e-5 without
+// this line too, so it decides who scores such a pair, not whether FP32 could).
 __host__ __device__ constexpr int long_max_bits(int rows) { return rows * 15 / 4; }
 constexpr int kLongTop = 100;             // a lane's bound for the coming steps, binary orders
 constexpr int kLongNone = -(1 << 28);     // exponent of "nothing there"
