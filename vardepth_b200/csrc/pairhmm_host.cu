@@ -1669,7 +1669,8 @@ int vd_forward(vd_engine* e, const vd_batch* b, const vd_params* p, double* out,
   // The first chunk is a quarter of the others: its host work and upload are
   // the only ones not hidden behind kernels.  Chunks run one after another on
   // the device, so each keeps at least kLongItemsPerWarp long-read items per
-  // warp (a chunk's last long items would otherwise run alone on the GPU).
+  // warp (a chunk's last long items would otherwise run alone on the GPU: measured
+  // with a warp per item, whose tail was longer than that of a warp per strip).
   constexpr int64_t kLongItemsPerWarp = 8;
   const int64_t pipeline_cells = (int64_t)(e->tuning.pipeline_gcells > 0 ? e->tuning.pipeline_gcells : 300) * 1'000'000'000LL;
   int64_t n_pipe = std::max<int64_t>(1, std::min<int64_t>(8, total_cells / pipeline_cells));

@@ -69,9 +69,9 @@ struct LongRows {
   uint32_t rb[R];        // read bases (kNeverBase for rows past the read)
   float miss[R];         // mismatch factor of rows 1 .. R-1 (the same for both halves)
   float hit[GEN ? R : 1];  // match factor (only where some row has P0 > P1; else 1)
-  float2 hit0, miss0;    // row 0's match and mismatch factors times the lane's boost, per half
+  float2 hit0, miss0;    // row 0's match and mismatch factors times the lane's scale against the lane above, per half
   float2 K[R], X[R];     // k1 f_i and (x/4) f_i (alpha f_n on the last row), both halves
-                         // (row 0's times the lane's boost)
+                         // (row 0's times that scale)
   float2 W[R], s[R];     // om of the next column and s of the column finished last
 };
 
